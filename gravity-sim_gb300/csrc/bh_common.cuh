@@ -158,14 +158,15 @@ inline int grid_for(uint64_t n, int threads) {
     return (int)b;
 }
 
-// Launch `kernel` on `st`.  With `pdl` the launch may begin while the previous kernel in
+// Launch `kernel` on `st` (with dynamic shared memory).  With `pdl` the launch may begin while the previous kernel in
 // the stream is still running; the kernel waits for it on entry (pdl_enter).
 template <typename... KArgs, typename... Args>
-cudaError_t launch(bool pdl, void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args... args) {
+cudaError_t launch_shared(bool pdl, void (*kernel)(KArgs...), dim3 grid, int block, unsigned shared_bytes,
+                          cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = shared_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -173,6 +174,11 @@ cudaError_t launch(bool pdl, void (*kernel)(KArgs...), int grid, int block, cuda
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch(bool pdl, void (*kernel)(KArgs...), dim3 grid, int block, cudaStream_t st, Args... args) {
+    return launch_shared(pdl, kernel, grid, block, 0u, st, args...);
 }
 
 // The same as a cooperative launch: every block of the grid is resident at once.

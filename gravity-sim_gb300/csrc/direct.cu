@@ -3,15 +3,17 @@
 // Replaces src/Simulation/Direct/Shaders/SimShader.comp:37-74 (one dispatch per step,
 // src/Simulation/Direct/DirectSimulation.cpp:306-319).
 //
-// FAST mode (k_direct_fast): each block owns an i-tile of 128*IPT particles and one
-// j-chunk; j is staged 64 at a time in shared memory as float4 {x, y, m, 0} (loaded as
-// float4 pairs of positions and float2 pairs of masses: j-tiles start at multiples of 64)
-// and broadcast to all threads; every thread keeps IPT targets in registers.  Each 64-wide
-// tile is summed plainly in FP32, and the tile partials are added with Kahan
-// compensation.  When the j-range is split over several blocks (small N, to fill 152
-// SMs), every block stores its compensated partial and the last block to finish an
-// i-tile (ticket counter, no waiting) combines the chunks in chunk order, again with
-// Kahan, and applies the integrator.  Results do not depend on block scheduling.
+// FAST mode: j is staged 64 sources at a time in shared memory (loaded as float4 pairs of
+// positions and float2 pairs of masses: j-tiles start at multiples of 64) and broadcast to
+// the threads, which keep their targets in registers.  Each 64-wide tile is summed plainly
+// in FP32, and the tile partials are added with Kahan compensation.
+//   k_direct_small  (N <= 8192) 32 targets per block, the tiles split over its 16 warps and
+//                   the warps' compensated sums added in shared memory
+//   k_direct_fast   (larger N) i-tiles of 128 threads with IPT targets each, j-chunks; every
+//                   block stores its compensated partial and the last block to finish an
+//                   i-tile (ticket counter, no waiting) adds the chunks in chunk order, again
+//                   with Kahan, and applies the integrator
+// Results do not depend on block scheduling.
 //
 // REFERENCE mode (k_direct_ref): one thread per particle, j ascending over all N_al
 // particles, plain FP32 accumulation and correctly rounded 1/sqrt -- the shader's order,
@@ -20,7 +22,7 @@
 // Roofline: 14 algorithmic FLOP per pair (2 sub, 2 FMA for r^2, rsqrt, 3 mul, 2 FMA),
 // 9 FP32 operations + 1 MUFU per pair, issued as packed f32x2 instructions for a thread's
 // two targets (4.5 issues + 1 MUFU per pair); FP32-bound.
-#include "internal.cuh"
+#include "bh_common.cuh"
 
 namespace gsim {
 namespace {
@@ -29,18 +31,71 @@ constexpr int kDirectBlock = 128;
 constexpr int kDirectTileJ = 64;
 constexpr int kDirectIpt = 2;  // default targets per thread (gs_shape.direct_targets: 2 or 4), in packed f32x2 pairs
 
-// Block (bx, by) of a system: i-tile bx, j-chunk by.  A plain launch passes blockIdx.x /
-// blockIdx.y, a batched launch the block's position inside its system's grid.  KAHAN
-// false (GS_FLAG_PLAIN_SUM) adds the tile partials and the chunks plainly, for the
-// precision study against the compensated sums.
-template <int IPT, bool KAHAN>
+// Steps launched programmatically behind one another (direct_step): wait for the step
+// before, then let the next one start.  In this order the next step's blocks start only once
+// the step before this one has finished: the step after next writes what that one read, and
+// its lines could otherwise still enter an L1 that the next step's start has already cleared.
+__device__ __forceinline__ void chain_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// 1/sqrt of a softened squared distance.  d2 >= eps2, so with a normal eps2 (FTZ) it is
+// never subnormal and the flush-to-zero form gives the same bits; the plain form also
+// scales subnormal inputs, six more instructions per pair of targets.
+template <bool FTZ>
+__device__ __forceinline__ float direct_rsqrt(float x) {
+    if (!FTZ) return rsqrtf(x);
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__host__ __device__ __forceinline__ bool direct_ftz(float eps2) { return eps2 >= 1.17549435e-38f; }
+
+// s + c carries the running sum (c: what the last additions lost); adds v to it.
+__device__ __forceinline__ void kahan_add(float v, float& s, float& c) {
+    const float y = v - c, u = s + y;
+    c = (u - s) - y;
+    s = u;
+}
+
+// Two consecutive sources (x, y, m pairs) on one target (P, Q: its position twice).  The
+// sources share packed f32x2 instructions up to the two sums, which take them in order:
+// dx, dy, d2 = fma(dx, dx, fma(dy, dy, eps2)), s = ((m r) r) r, t += d s, each lane rounding
+// like the scalar instruction.
+template <bool FTZ>
+__device__ __forceinline__ void tile_pair(float2 x, float2 y, float2 m, float2 P, float2 Q, float2 E2, float& tx,
+                                          float& ty) {
+    const float2 dx = sub2(x, P), dy = sub2(y, Q);
+    const float2 d2 = fma2(dx, dx, fma2(dy, dy, E2));
+    const float2 r = make_float2(direct_rsqrt<FTZ>(d2.x), direct_rsqrt<FTZ>(d2.y));
+    const float2 s = mul2(mul2(mul2(m, r), r), r);
+    tx = fmaf(dx.x, s.x, tx);
+    ty = fmaf(dy.x, s.x, ty);
+    tx = fmaf(dx.y, s.y, tx);
+    ty = fmaf(dy.y, s.y, ty);
+}
+
+// Block (bx, by) of a large system: 128 IPT targets (i-tile bx), j-chunk by.  A plain launch
+// passes blockIdx.x / blockIdx.y, a batched launch the block's position inside its system's
+// grid.  KAHAN false (GS_FLAG_PLAIN_SUM) adds the tile partials and the chunks plainly, for
+// the precision study against the compensated sums.
+//
+// The loop is bound by the FMA pipe (9 packed operations of two cycles for a source and two
+// targets) next to the 16 cycles that two MUFU instructions take: 18 of about 23.5 cycles a
+// source.  N = 50,000: 964 us a step with the rsqrt form that scales subnormal inputs, a tile
+// loaded between two barriers and chunks for one set of resident blocks; 738 us with the
+// flush-to-zero form, the next tile in flight and two sets (the shorter chunks even out the
+// tail).  Eight targets per thread (112 registers) took 861 us, equal contiguous runs of
+// (target group, tile) units per block 827 us.
+template <int IPT, bool KAHAN, bool FTZ>
 __device__ __forceinline__ void direct_fast_body(uint32_t bx, uint32_t by, const float2* __restrict__ pos,
                                                  const float2* __restrict__ vel, const float* __restrict__ mass,
                                                  float2* __restrict__ pos_out, float2* __restrict__ vel_out,
                                                  float2* __restrict__ acc_rec, uint32_t n_al, int chunks,
                                                  uint32_t jchunk, float eps2, float k, float hdt,
                                                  float4* __restrict__ partials, uint32_t* __restrict__ tickets) {
-    __shared__ float4 sj[kDirectTileJ];
+    __shared__ float4 sj[2][kDirectTileJ];
     __shared__ uint32_t s_ticket;
     const int t = threadIdx.x;
     const uint32_t tile_base = bx * (kDirectBlock * IPT);
@@ -66,13 +121,26 @@ __device__ __forceinline__ void direct_fast_body(uint32_t bx, uint32_t by, const
     }
     const float2 E2 = make_float2(eps2, eps2);
 
-    for (uint32_t jt = j0; jt < j1; jt += kDirectTileJ) {
-        __syncthreads();
-        if (t < kDirectTileJ / 2) {  // one float4 of two positions and one float2 of their masses per thread
-            const float4 q = reinterpret_cast<const float4*>(pos)[(jt >> 1) + t];
-            const float2 m = reinterpret_cast<const float2*>(mass)[(jt >> 1) + t];
-            sj[2 * t] = make_float4(q.x, q.y, m.x, 0.f);
-            sj[2 * t + 1] = make_float4(q.z, q.w, m.y, 0.f);
+    // the first half of the threads stage a tile: one float4 of two positions and one float2
+    // of their masses each, loaded while the tile before is summed
+    const bool stage = t < kDirectTileJ / 2;
+    const float4* pos2 = reinterpret_cast<const float4*>(pos) + t;
+    const float2* mass2 = reinterpret_cast<const float2*>(mass) + t;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 m = make_float2(0.f, 0.f);
+    if (stage) {
+        q = pos2[j0 >> 1];
+        m = mass2[j0 >> 1];
+    }
+    int buf = 0;
+    for (uint32_t jt = j0; jt < j1; jt += kDirectTileJ, buf ^= 1) {
+        if (stage) {  // the other buffer's readers passed the barrier of the tile before
+            sj[buf][2 * t] = make_float4(q.x, q.y, m.x, 0.f);
+            sj[buf][2 * t + 1] = make_float4(q.z, q.w, m.y, 0.f);
+            if (jt + kDirectTileJ < j1) {
+                q = pos2[(jt + kDirectTileJ) >> 1];
+                m = mass2[(jt + kDirectTileJ) >> 1];
+            }
         }
         __syncthreads();
         // Pairs of the thread's targets share packed f32x2 instructions (each lane rounds
@@ -83,40 +151,27 @@ __device__ __forceinline__ void direct_fast_body(uint32_t bx, uint32_t by, const
         for (int h = 0; h < NP; ++h) tx2[h] = ty2[h] = make_float2(0.f, 0.f);
 #pragma unroll 16
         for (int jj = 0; jj < kDirectTileJ; ++jj) {
-            const float4 q = sj[jj];
+            const float4 g = sj[buf][jj];
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
-                const float2 dx = sub2(make_float2(q.x, q.x), P2[h]), dy = sub2(make_float2(q.y, q.y), Q2[h]);
+                const float2 dx = sub2(make_float2(g.x, g.x), P2[h]), dy = sub2(make_float2(g.y, g.y), Q2[h]);
                 const float2 d2 = fma2(dx, dx, fma2(dy, dy, E2));
-                const float2 rr = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
-                const float2 s = mul2(mul2(mul2(make_float2(q.z, q.z), rr), rr), rr);
+                const float2 rr = make_float2(direct_rsqrt<FTZ>(d2.x), direct_rsqrt<FTZ>(d2.y));
+                const float2 s = mul2(mul2(mul2(make_float2(g.z, g.z), rr), rr), rr);
                 tx2[h] = fma2(dx, s, tx2[h]);
                 ty2[h] = fma2(dy, s, ty2[h]);
             }
         }
-        float tx[IPT], ty[IPT];
-#pragma unroll
-        for (int h = 0; h < NP; ++h) {
-            tx[2 * h] = tx2[h].x;
-            tx[2 * h + 1] = tx2[h].y;
-            ty[2 * h] = ty2[h].x;
-            ty[2 * h + 1] = ty2[h].y;
-        }
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {  // Kahan-compensated add of the tile partial
+            const float tx = r & 1 ? tx2[r / 2].y : tx2[r / 2].x, ty = r & 1 ? ty2[r / 2].y : ty2[r / 2].x;
             if (!KAHAN) {
-                sx[r] += tx[r];
-                sy[r] += ty[r];
+                sx[r] += tx;
+                sy[r] += ty;
                 continue;
             }
-            float y = tx[r] - cx[r];
-            float u = sx[r] + y;
-            cx[r] = (u - sx[r]) - y;
-            sx[r] = u;
-            y = ty[r] - cy[r];
-            u = sy[r] + y;
-            cy[r] = (u - sy[r]) - y;
-            sy[r] = u;
+            kahan_add(tx, sx[r], cx[r]);
+            kahan_add(ty, sy[r], cy[r]);
         }
     }
 
@@ -137,21 +192,16 @@ __device__ __forceinline__ void direct_fast_body(uint32_t bx, uint32_t by, const
             uint32_t i = tile_base + t + r * kDirectBlock;
             float ax = 0.f, ay = 0.f, kx = 0.f, ky = 0.f;
             if (i < n_al) {
+#pragma unroll 8
                 for (int c = 0; c < chunks; ++c) {
-                    float4 q = __ldcg(&partials[(size_t)c * n_al + i]);
+                    const float4 pc = __ldcg(&partials[(size_t)c * n_al + i]);
                     if (!KAHAN) {
-                        ax += q.x;
-                        ay += q.y;
+                        ax += pc.x;
+                        ay += pc.y;
                         continue;
                     }
-                    float y = (q.x - q.z) - kx;
-                    float u = ax + y;
-                    kx = (u - ax) - y;
-                    ax = u;
-                    y = (q.y - q.w) - ky;
-                    u = ay + y;
-                    ky = (u - ay) - y;
-                    ay = u;
+                    kahan_add(pc.x - pc.z, ax, kx);
+                    kahan_add(pc.y - pc.w, ay, ky);
                 }
             }
             sx[r] = ax;
@@ -173,6 +223,110 @@ __device__ __forceinline__ void direct_fast_body(uint32_t bx, uint32_t by, const
         pos_out[i] = make_float2(fmaf(v.x + nvx, hdt, px[r]), fmaf(v.y + nvy, hdt, py[r]));  // :69
         vel_out[i] = make_float2(nvx, nvy);
     }
+}
+
+// A small system: 32 targets per block, one per lane, and the 64-wide source tiles split over
+// the block's W warps.  Part p of min(16, K) parts holds tiles [p K / P, (p + 1) K / P) and
+// is summed by warp p mod W with Kahan compensation; the parts are then added in part order
+// in shared memory, again with Kahan.  The parts do not depend on W, so it changes no bit.
+// What bounds a small system is latency (a block's chain of tile loads and sums) and the
+// number of warps: N = 4096 as 16 i-tiles x 16 j-chunks of 128-thread blocks, combined
+// through global partials by the last block, kept 1.7 warps per scheduler busy and took
+// 20.6 us a step; 128 blocks of 16 warps, each staging its own tiles without a block barrier,
+// 10.4 us (N = 1024: 16.5 -> 6.2 us, N = 8192: 41.2 -> 30.9 us).  The tiles are staged as
+// separate x, y and m arrays so that two consecutive sources share packed instructions.
+// Beyond kDirectSmallMax the 4-byte-per-lane broadcasts of one target per lane bound the
+// loop (three 16-byte shared loads per four sources and 32 targets), and the large-system
+// kernel is faster (N = 12288: 65.5 us here).
+constexpr uint32_t kDirectParts = 16;
+constexpr uint32_t kDirectSmallMax = 12288;
+constexpr int kDirectSmallWarps = 16;
+
+template <int W>
+struct DirectSmallSmem {
+    float x[W][kDirectTileJ], y[W][kDirectTileJ], m[W][kDirectTileJ];
+    float4 part[kDirectParts][32];  // {sx, sy, cx, cy}
+};
+
+template <int W, bool KAHAN, bool FTZ>
+__device__ __forceinline__ void direct_small_body(DirectSmallSmem<W>& g, uint32_t bx, const float2* __restrict__ pos,
+                                                  const float2* __restrict__ vel, const float* __restrict__ mass,
+                                                  float2* __restrict__ pos_out, float2* __restrict__ vel_out,
+                                                  float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float k,
+                                                  float hdt) {
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t tiles = n_al / kDirectTileJ, parts = min(kDirectParts, tiles);
+    const uint32_t i = bx * 32 + lane;  // n_al is a multiple of 64: every target exists
+    const float2 p = pos[i];
+    const float2 P = make_float2(p.x, p.x), Q = make_float2(p.y, p.y), E2 = make_float2(eps2, eps2);
+    const float4* X = reinterpret_cast<const float4*>(g.x[w]);
+    const float4* Y = reinterpret_cast<const float4*>(g.y[w]);
+    const float4* M = reinterpret_cast<const float4*>(g.m[w]);
+    for (uint32_t part = w; part < parts; part += W) {
+        const uint32_t t0 = part * tiles / parts, t1 = (part + 1) * tiles / parts;
+        float sx = 0.f, sy = 0.f, cx = 0.f, cy = 0.f;
+        float4 q = reinterpret_cast<const float4*>(pos)[t0 * 32 + lane];  // two positions and their masses
+        float2 m = reinterpret_cast<const float2*>(mass)[t0 * 32 + lane];
+        for (uint32_t jt = t0; jt < t1; ++jt) {
+            __syncwarp();
+            reinterpret_cast<float2*>(g.x[w])[lane] = make_float2(q.x, q.z);
+            reinterpret_cast<float2*>(g.y[w])[lane] = make_float2(q.y, q.w);
+            reinterpret_cast<float2*>(g.m[w])[lane] = m;
+            __syncwarp();
+            if (jt + 1 < t1) {  // in flight while this tile is summed
+                q = reinterpret_cast<const float4*>(pos)[(jt + 1) * 32 + lane];
+                m = reinterpret_cast<const float2*>(mass)[(jt + 1) * 32 + lane];
+            }
+            float tx = 0.f, ty = 0.f;
+#pragma unroll
+            for (int jj = 0; jj < kDirectTileJ / 4; ++jj) {
+                const float4 x4 = X[jj], y4 = Y[jj], m4 = M[jj];
+                tile_pair<FTZ>(make_float2(x4.x, x4.y), make_float2(y4.x, y4.y), make_float2(m4.x, m4.y), P, Q, E2, tx,
+                               ty);
+                tile_pair<FTZ>(make_float2(x4.z, x4.w), make_float2(y4.z, y4.w), make_float2(m4.z, m4.w), P, Q, E2, tx,
+                               ty);
+            }
+            if (KAHAN) {
+                kahan_add(tx, sx, cx);
+                kahan_add(ty, sy, cy);
+            } else {
+                sx += tx;
+                sy += ty;
+            }
+        }
+        g.part[part][lane] = make_float4(sx, sy, cx, cy);
+    }
+    __syncthreads();
+    if (w) return;
+    float ax = 0.f, ay = 0.f, kx = 0.f, ky = 0.f;
+    for (uint32_t part = 0; part < parts; ++part) {
+        const float4 q = g.part[part][lane];
+        if (KAHAN) {
+            kahan_add(q.x - q.z, ax, kx);
+            kahan_add(q.y - q.w, ay, ky);
+        } else {
+            ax += q.x;
+            ay += q.y;
+        }
+    }
+    ax -= kx;
+    ay -= ky;
+    if (acc_rec) acc_rec[i] = make_float2(ax, ay);
+    const float2 v = vel[i];
+    const float nvx = fmaf(ax, k, v.x), nvy = fmaf(ay, k, v.y);  // SimShader.comp:68
+    pos_out[i] = make_float2(fmaf(v.x + nvx, hdt, p.x), fmaf(v.y + nvy, hdt, p.y));  // :69
+    vel_out[i] = make_float2(nvx, nvy);
+}
+
+template <bool KAHAN, bool FTZ>
+__global__ void __launch_bounds__(kDirectSmallWarps * 32)
+k_direct_small(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
+               float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
+               uint32_t n_al, float eps2, float k, float hdt) {
+    chain_enter();
+    __shared__ __align__(16) DirectSmallSmem<kDirectSmallWarps> g;
+    direct_small_body<kDirectSmallWarps, KAHAN, FTZ>(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2,
+                                                     k, hdt);
 }
 
 __device__ __forceinline__ void direct_ref_body(uint32_t bx, const float2* __restrict__ pos,
@@ -207,26 +361,28 @@ __device__ __forceinline__ void direct_ref_body(uint32_t bx, const float2* __res
     vel_out[i] = make_float2(nvx, nvy);
 }
 
-template <int IPT, bool KAHAN>
+template <int IPT, bool KAHAN, bool FTZ>
 __global__ void __launch_bounds__(kDirectBlock)
 k_direct_fast(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
               float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
-              uint32_t n_al, int chunks, uint32_t jchunk, float eps2, float k, float hdt,
-              float4* __restrict__ partials, uint32_t* __restrict__ tickets) {
-    direct_fast_body<IPT, KAHAN>(blockIdx.x, blockIdx.y, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, chunks, jchunk,
-                          eps2, k, hdt, partials, tickets);
+              uint32_t n_al, int chunks, uint32_t jchunk, float eps2, float k, float hdt, float4* __restrict__ partials,
+              uint32_t* __restrict__ tickets) {
+    chain_enter();
+    direct_fast_body<IPT, KAHAN, FTZ>(blockIdx.x, blockIdx.y, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, chunks,
+                                      jchunk, eps2, k, hdt, partials, tickets);
 }
 
 __global__ void __launch_bounds__(64)
 k_direct_ref(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
              float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
              uint32_t n_al, float eps2, float k, float hdt) {
+    chain_enter();
     direct_ref_body(blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
 }
 
 // Batched direct sum: one launch over every direct-sum system of a plan.  Block b belongs
-// to the system whose table range holds it; inside the system it is block (b mod i-tiles,
-// b div i-tiles) of the plain grid, so each system sums in the plain order.
+// to the system whose table range holds it and does the work of the plain launch's block of
+// that index (small systems on four warps per block instead of sixteen, which changes no bit).
 __device__ __forceinline__ uint32_t direct_batch_sys(const uint32_t* __restrict__ first, uint32_t nsys,
                                                      uint32_t b) {
     uint32_t lo = 0, hi = nsys;
@@ -238,19 +394,33 @@ __device__ __forceinline__ uint32_t direct_batch_sys(const uint32_t* __restrict_
     return lo;
 }
 
+template <int IPT, bool KAHAN, bool FTZ>
+__device__ __forceinline__ void direct_batch_body(DirectSmallSmem<kDirectBlock / 32>& g, const SysDesc& d, uint32_t b,
+                                                  int in, int out) {
+    if (!d.chunks)
+        direct_small_body<kDirectBlock / 32, KAHAN, FTZ>(g, b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out],
+                                                         d.acc, d.n_al, d.eps2, d.k, d.hdt);
+    else
+        direct_fast_body<IPT, KAHAN, FTZ>(b % d.itiles, b / d.itiles, d.pos[in], d.vel[in], d.mass[in], d.pos[out],
+                                          d.vel[out], d.acc, d.n_al, (int)d.chunks, d.jchunk, d.eps2, d.k, d.hdt,
+                                          d.partials, d.tickets);
+}
+
 template <bool EXACT, bool KAHAN, int IPT>
-__global__ void __launch_bounds__(EXACT ? 64 : kDirectBlock)
+__global__ void __launch_bounds__(EXACT ? 64 : kDirectBlock, IPT == 4 ? 6 : 8)
 kb_direct(const SysDesc* __restrict__ descs, const uint32_t* __restrict__ first, uint32_t nsys, uint32_t step) {
     const uint32_t s = direct_batch_sys(first, nsys, blockIdx.x);
     const SysDesc& d = descs[s];
     const uint32_t b = blockIdx.x - __ldg(&first[s]);
     const int in = (int)((d.parity + step) & 1u), out = in ^ 1;
-    if (EXACT)
+    if constexpr (EXACT) {
         direct_ref_body(b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.k,
                         d.hdt);
-    else
-        direct_fast_body<IPT, KAHAN>(b % d.itiles, b / d.itiles, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out],
-                            d.acc, d.n_al, (int)d.chunks, d.jchunk, d.eps2, d.k, d.hdt, d.partials, d.tickets);
+    } else {
+        __shared__ __align__(16) DirectSmallSmem<kDirectBlock / 32> g;
+        if (direct_ftz(d.eps2)) direct_batch_body<IPT, KAHAN, true>(g, d, b, in, out);
+        else direct_batch_body<IPT, KAHAN, false>(g, d, b, in, out);
+    }
 }
 
 __global__ void __launch_bounds__(256)
@@ -361,11 +531,39 @@ static int pick_chunks(uint64_t n_al, int ipt, uint32_t blocks_per_sm) {
     return (int)c;
 }
 
+// one ticket per i-tile of two targets per thread, the smallest
+static uint64_t direct_tickets(uint64_t n_al) { return (n_al + kDirectBlock * 2 - 1) / (kDirectBlock * 2); }
+
+// The j-split of a system: chunks of jchunk sources (a multiple of 64); chunks 0: a small
+// system (k_direct_small).  Enough chunks for blocks_per_sm blocks of four targets per thread
+// on every SM (twice as many blocks of two), at least 512 sources in each and at most
+// max_chunks (the scratch's rows).
+struct DirectGrid {
+    uint32_t chunks, jchunk;
+};
+static uint32_t pick_rows(uint64_t n_al, uint32_t blocks_per_sm) {
+    if (n_al <= kDirectSmallMax) return 0;
+    const uint64_t itiles = (n_al + kDirectBlock * 4 - 1) / (kDirectBlock * 4), want = 152ull * blocks_per_sm;
+    uint64_t c = (want + itiles - 1) / itiles;
+    if (c > n_al / 512) c = n_al / 512;
+    return (uint32_t)(c < 1 ? 1 : c > 64 ? 64 : c);
+}
+static DirectGrid pick_grid(uint64_t n_al, uint32_t blocks_per_sm, uint32_t max_chunks) {
+    DirectGrid g{};
+    uint64_t c = pick_rows(n_al, blocks_per_sm);
+    if (!c) return g;
+    if (c > max_chunks) c = max_chunks;
+    const uint64_t j = (n_al + c - 1) / c;
+    g.jchunk = (uint32_t)((j + kDirectTileJ - 1) / kDirectTileJ * kDirectTileJ);
+    g.chunks = (uint32_t)((n_al + g.jchunk - 1) / g.jchunk);
+    return g;
+}
+
 static int shape_ipt(const gs_shape& sh) { return sh.direct_targets == 4 ? 4 : 2; }
 
-// Lays the j-chunk partials and tickets out in the system's slab (sizing pass: counts):
-// for the chunks of the creation shape with either targets-per-thread value, tickets for
-// the most i-tiles (2 targets per thread).
+// Lays the j-chunk partials and tickets out in the system's slab (sizing pass: counts), for
+// the j-split of the creation shape.  direct_max_chunks keeps gs_set_shape's limit: a shape
+// may ask for no finer split than one laid out by pick_chunks would hold.
 void direct_carve(gs_sim* s) {
     DirectWork& w = s->dw;
     w.ipt = shape_ipt(s->shape);
@@ -375,10 +573,10 @@ void direct_carve(gs_sim* s) {
     s->direct_max_chunks = (uint32_t)(c2 > c4 ? c2 : c4);
     w.partials = nullptr;
     w.tickets = nullptr;
-    if (s->direct_max_chunks > 1) {
-        const uint64_t itiles = (s->n_al + kDirectBlock * 2 - 1) / (kDirectBlock * 2);
-        sim_carve(s, (void**)&w.partials, sizeof(float4) * s->n_al * (size_t)s->direct_max_chunks);
-        sim_carve(s, (void**)&w.tickets, sizeof(uint32_t) * itiles);
+    w.rows = pick_rows(s->n_al, s->shape.direct_blocks_per_sm);
+    if (w.rows > 1) {
+        sim_carve(s, (void**)&w.partials, sizeof(float4) * s->n_al * (size_t)w.rows);
+        sim_carve(s, (void**)&w.tickets, sizeof(uint32_t) * direct_tickets(s->n_al));
     }
 }
 
@@ -389,58 +587,67 @@ uint32_t direct_chunks_needed(const gs_sim* s, const gs_shape& sh) {
 cudaError_t direct_init(gs_sim* s) {
     const DirectWork& w = s->dw;
     if (!w.tickets) return cudaSuccess;
-    const uint64_t itiles = (s->n_al + kDirectBlock * 2 - 1) / (kDirectBlock * 2);
-    return cudaMemsetAsync(w.tickets, 0, sizeof(uint32_t) * itiles, s->stream);
+    return cudaMemsetAsync(w.tickets, 0, sizeof(uint32_t) * direct_tickets(s->n_al), s->stream);
 }
 
-// Grid of k_direct_fast for `ipt` targets per thread: i-tiles x j-chunks, each chunk a
-// multiple of 64 sources.  The chunks come from the system's own shape, so a system sums
-// in the same order whichever targets per thread run it (alone or in a batch).
-static void direct_grid(const gs_sim* s, int ipt, uint32_t& itiles, uint32_t& jchunk, uint32_t& chunks) {
-    const uint32_t n_al = (uint32_t)s->n_al;
-    const uint32_t c = direct_chunks_needed(s, s->shape);
-    itiles = (n_al + kDirectBlock * ipt - 1) / (kDirectBlock * ipt);
-    jchunk = (n_al + c - 1) / c;
-    jchunk = (jchunk + kDirectTileJ - 1) / kDirectTileJ * kDirectTileJ;
-    chunks = (n_al + jchunk - 1) / jchunk;
+// How a system splits its sum: from its own shape, so that it sums in the same order
+// whichever targets per thread run it (alone or in a batch).
+static DirectGrid direct_grid(const gs_sim* s) {
+    return pick_grid(s->n_al, s->shape.direct_blocks_per_sm, s->dw.rows);
+}
+static uint32_t direct_itiles(uint64_t n_al, int ipt) { return (uint32_t)((n_al + kDirectBlock * ipt - 1) / (kDirectBlock * ipt)); }
+
+// The fast kernels' launch; every array as the kernels take it.  pdl: the launch may begin
+// while the step before it still runs (the kernels wait for it on entry).
+static cudaError_t direct_fast_launch(bool pdl, const DirectGrid& d, int ipt, bool plain, const float2* pos,
+                                      const float2* vel, const float* mass, float2* pos_out, float2* vel_out,
+                                      float2* acc, uint32_t n_al, float eps2, float k, float hdt, float4* partials,
+                                      uint32_t* tickets, cudaStream_t st) {
+    const bool ftz = direct_ftz(eps2);
+    if (!d.chunks) {
+        auto fn = plain ? (ftz ? k_direct_small<false, true> : k_direct_small<false, false>)
+                        : (ftz ? k_direct_small<true, true> : k_direct_small<true, false>);
+        return launch(pdl, fn, dim3(n_al / 32), kDirectSmallWarps * 32, st, pos, vel, mass, pos_out, vel_out, acc,
+                      n_al, eps2, k, hdt);
+    }
+    auto fn = plain ? (ftz ? (ipt == 4 ? k_direct_fast<4, false, true> : k_direct_fast<2, false, true>)
+                           : (ipt == 4 ? k_direct_fast<4, false, false> : k_direct_fast<2, false, false>))
+                    : (ftz ? (ipt == 4 ? k_direct_fast<4, true, true> : k_direct_fast<2, true, true>)
+                           : (ipt == 4 ? k_direct_fast<4, true, false> : k_direct_fast<2, true, false>));
+    return launch(pdl, fn, dim3(direct_itiles(n_al, ipt), d.chunks), kDirectBlock, st, pos, vel, mass, pos_out, vel_out,
+                  acc, n_al, (int)d.chunks, d.jchunk, eps2, k, hdt, partials, tickets);
 }
 
-cudaError_t direct_step(gs_sim* s, int in, int out, bool profile) {
+cudaError_t direct_step(gs_sim* s, int in, int out, bool profile, bool chained) {
     const float k = s->dt_eff * s->G;  // SimShader.comp:68 (SIMULATION_TIME * GRAVITATIONAL_CONST)
     const float hdt = 0.5f * s->dt_eff;
     const uint32_t n_al = (uint32_t)s->n_al;
+    const bool pdl = chained && !profile;
+    cudaError_t e;
     stage_begin(s, kStageDirect, profile);
-    if (s->p.math_mode == GS_MATH_REFERENCE) {
-        k_direct_ref<<<n_al / 64, 64, 0, s->stream>>>(s->pos[in], s->vel[in], s->mass[in], s->pos[out],
-                                                       s->vel[out], s->acc, n_al, s->eps2, k, hdt);
-    } else {
-        DirectWork& w = s->dw;
-        const int ipt = shape_ipt(s->shape);
-        uint32_t itiles, jchunk, chunks;
-        direct_grid(s, ipt, itiles, jchunk, chunks);
-        dim3 grid(itiles, chunks);
-        const bool plain = (s->p.flags & GS_FLAG_PLAIN_SUM) != 0;
-        auto fn = ipt == 4 ? (plain ? k_direct_fast<4, false> : k_direct_fast<4, true>)
-                           : (plain ? k_direct_fast<2, false> : k_direct_fast<2, true>);
-        fn<<<grid, kDirectBlock, 0, s->stream>>>(s->pos[in], s->vel[in], s->mass[in], s->pos[out], s->vel[out],
-                                                  s->acc, n_al, (int)chunks, jchunk, s->eps2, k, hdt, w.partials,
-                                                  w.tickets);
-    }
+    if (s->p.math_mode == GS_MATH_REFERENCE)
+        e = launch(pdl, k_direct_ref, dim3(n_al / 64), 64, s->stream, s->pos[in], s->vel[in],
+                   s->mass[in], s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k, hdt);
+    else
+        e = direct_fast_launch(pdl, direct_grid(s), shape_ipt(s->shape), (s->p.flags & GS_FLAG_PLAIN_SUM) != 0,
+                               s->pos[in], s->vel[in], s->mass[in], s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k,
+                               hdt, s->dw.partials, s->dw.tickets, s->stream);
     count_launch(s);
     stage_end(s, kStageDirect, profile);
-    return cudaGetLastError();
+    return e;
 }
 
 void direct_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& batch_shape) {
     for (int t = 0; t < kTabCount; ++t) blocks[t] = 0;
-    uint32_t itiles, jchunk, chunks;
-    direct_grid(s, shape_ipt(batch_shape), itiles, jchunk, chunks);
-    d.itiles = itiles;
-    d.jchunk = jchunk;
-    d.chunks = chunks;
+    const DirectGrid g = direct_grid(s);
+    d.itiles = direct_itiles(s->n_al, shape_ipt(batch_shape));
+    d.chunks = g.chunks;
+    d.jchunk = g.jchunk;
     d.partials = s->dw.partials;
     d.tickets = s->dw.tickets;
-    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? (uint32_t)(s->n_al / 64) : itiles * chunks;
+    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? (uint32_t)(s->n_al / 64)
+                         : g.chunks                          ? d.itiles * g.chunks
+                                                             : (uint32_t)(s->n_al / 32);
 }
 
 cudaError_t direct_batch_step(const BatchPlan& p, uint32_t step, cudaStream_t st) {
@@ -480,7 +687,7 @@ namespace gsim {
 namespace {
 
 constexpr size_t kNoAllocPartialBytes = 4u << 20;  // j-chunk partials, 4 MiB
-constexpr uint32_t kNoAllocMaxTiles = GS_NOALLOC_MAX_PARTICLES / (kDirectBlock * 2);
+constexpr uint32_t kNoAllocMaxTiles = GS_NOALLOC_MAX_PARTICLES / 256;
 
 static __device__ __align__(256) float4 g_noalloc_partials[kNoAllocPartialBytes / sizeof(float4)];
 static __device__ __align__(256) uint32_t g_noalloc_tickets[kNoAllocMaxTiles];
@@ -528,28 +735,23 @@ extern "C" gs_status gs_direct_step_noalloc(const float* d_pos_in, const float* 
                   "of its built-in scratch; use gs_create / gs_run for larger systems");
         return GS_ERR_CAPACITY;
     }
+    const uint32_t n_al = (uint32_t)n;
+    const uint32_t fit = (uint32_t)(kNoAllocPartialBytes / (sizeof(float4) * n_al));  // >= 4 for n <= 65536
+    const DirectGrid split = pick_grid(n_al, 12, fit);
+    cudaStream_t s = (cudaStream_t)stream;
     float4* partials = nullptr;
     uint32_t* tickets = nullptr;
-    gs_status st = noalloc_scratch(&partials, &tickets);
-    if (st != GS_OK) return st;
-
-    const uint32_t n_al = (uint32_t)n;
-    const uint32_t itiles = (n_al + kDirectBlock * kDirectIpt - 1) / (kDirectBlock * kDirectIpt);
-    int chunks = pick_chunks(n_al, kDirectIpt, 12);
-    const int fit = (int)(kNoAllocPartialBytes / (sizeof(float4) * n_al));  // >= 4 for n <= 65536
-    if (chunks > fit) chunks = fit;
-    uint32_t jchunk = (n_al + chunks - 1) / chunks;
-    jchunk = (jchunk + kDirectTileJ - 1) / kDirectTileJ * kDirectTileJ;
-    chunks = (int)((n_al + jchunk - 1) / jchunk);
-    cudaStream_t s = (cudaStream_t)stream;
-    // the tickets must start at zero; the array keeps whatever the previous call left
-    if (chunks > 1) GS_CUDA(cudaMemsetAsync(tickets, 0, itiles * sizeof(uint32_t), s));
+    if (split.chunks > 1) {  // small systems need no scratch
+        gs_status st = noalloc_scratch(&partials, &tickets);
+        if (st != GS_OK) return st;
+        // the tickets must start at zero; the array keeps whatever the previous call left
+        GS_CUDA(cudaMemsetAsync(tickets, 0, direct_tickets(n_al) * sizeof(uint32_t), s));
+    }
     const float eps2 = softening_len * softening_len;
     const float k = simulation_time * gravitational_const;
     const float hdt = 0.5f * simulation_time;
-    k_direct_fast<kDirectIpt, true><<<dim3(itiles, chunks), kDirectBlock, 0, s>>>(
-        (const float2*)d_pos_in, (const float2*)d_vel_in, d_mass, (float2*)d_pos_out, (float2*)d_vel_out, nullptr,
-        n_al, chunks, jchunk, eps2, k, hdt, partials, tickets);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(direct_fast_launch(false, split, kDirectIpt, false, (const float2*)d_pos_in, (const float2*)d_vel_in, d_mass,
+                               (float2*)d_pos_out, (float2*)d_vel_out, nullptr, n_al, eps2, k, hdt, partials, tickets,
+                               s));
     return GS_OK;
 }

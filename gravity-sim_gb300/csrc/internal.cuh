@@ -152,8 +152,9 @@ struct BHWork {
 struct DirectWork {
     int ipt = 2;           // particles per thread of the creation shape
     int block = 128;       // threads per block
-    float4* partials = nullptr;  // [direct_max_chunks][N_al] {sx, sy, cx, cy}
+    float4* partials = nullptr;  // [rows][N_al] {sx, sy, cx, cy}
     uint32_t* tickets = nullptr; // [i-tiles]
+    uint32_t rows = 0;           // j-chunks the partials hold (0, 1: no partials)
 };
 
 // One system of a batch as the batched stage kernels see it: its buffers (both ping-pong
@@ -201,7 +202,7 @@ struct SysDesc {
     // direct sum (DirectWork)
     float4* partials;
     uint32_t* tickets;
-    uint32_t itiles, chunks, jchunk;
+    uint32_t itiles, chunks, jchunk;  // chunks 0: a small system (k_direct_small)
 };
 
 // Per-stage block tables of a batch: table t holds the exclusive prefix of the blocks each
@@ -312,7 +313,8 @@ cudaError_t bh_init(gs_sim* s);
 cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate);
 void direct_carve(gs_sim* s);
 cudaError_t direct_init(gs_sim* s);
-cudaError_t direct_step(gs_sim* s, int in, int out, bool profile);
+// chained: the launch directly follows another step's on the stream
+cudaError_t direct_step(gs_sim* s, int in, int out, bool profile, bool chained);
 cudaError_t accel_f64(gs_sim* s, uint32_t n_targets, const uint32_t* d_targets, double2* d_out);
 gs_status energy_f64(gs_sim* s, double* kinetic, double* potential);
 void free_snapshot_ring(const gs_sim* s);

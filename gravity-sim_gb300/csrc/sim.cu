@@ -302,10 +302,10 @@ gs_status upload(gs_sim* s, const float* pos, const float* vel, const float* mas
     return sim_wait(s);
 }
 
-cudaError_t enqueue_step(gs_sim* s, int in, bool profile, bool estimate) {
+cudaError_t enqueue_step(gs_sim* s, int in, bool profile, bool estimate, bool chained = false) {
     const int out = in ^ 1;
     if (s->p.algorithm == GS_BARNES_HUT) return bh_step(s, in, out, profile, estimate);
-    return direct_step(s, in, out, profile);
+    return direct_step(s, in, out, profile, chained);
 }
 
 // The next step has to estimate |a| first: the relative criterion with no previous |a|
@@ -495,7 +495,10 @@ gs_status gs_run(gs_sim* s, uint32_t count) {
     }
     if (!count) return GS_OK;
     const bool profile = (s->p.flags & GS_FLAG_PROFILE) != 0;
-    const bool graphs = !(s->p.flags & GS_FLAG_NO_GRAPH);
+    // A direct-sum step is one kernel: launched as it is, each step after the first
+    // programmatically behind the one before it (a graph launch per step left 2.4 us between
+    // the kernels of a 1024-particle system, and its capture lengthened the first run).
+    const bool graphs = !(s->p.flags & GS_FLAG_NO_GRAPH) && s->p.algorithm == GS_BARNES_HUT;
     for (uint32_t c = 0; c < count; ++c) {
         const int in = s->in;
         if (s->profile_pending) {  // the previous step's stage events are about to be re-recorded
@@ -530,7 +533,7 @@ gs_status gs_run(gs_sim* s, uint32_t count) {
             s->kernel_launches += s->launches_per_step[gi];
         } else {
             s->launches_in_step = 0;
-            GS_CUDA(enqueue_step(s, in, profile, est));
+            GS_CUDA(enqueue_step(s, in, profile, est, c > 0));
             s->kernel_launches += s->launches_in_step;
         }
         s->amag_known = true;  // this step leaves every particle's |a|
