@@ -15,9 +15,9 @@
 //                   with Kahan, and applies the integrator
 // Results do not depend on block scheduling.
 //
-// REFERENCE mode (k_direct_ref): one thread per particle, j ascending over all N_al
-// particles, plain FP32 accumulation and correctly rounded 1/sqrt -- the shader's order,
-// bit-identical to the CPU restatement.
+// REFERENCE mode (k_direct_ref): j ascending over all N_al particles, plain FP32
+// accumulation and correctly rounded 1/sqrt -- the shader's order, bit-identical to the CPU
+// restatement; the factors of the terms are made ahead of the sums by other warps.
 //
 // Roofline: 14 algorithmic FLOP per pair (2 sub, 2 FMA for r^2, rsqrt, 3 mul, 2 FMA),
 // 9 FP32 operations + 1 MUFU per pair, issued as packed f32x2 instructions for a thread's
@@ -329,34 +329,169 @@ k_direct_small(const float2* __restrict__ pos, const float2* __restrict__ vel, c
                                                      k, hdt);
 }
 
-__device__ __forceinline__ void direct_ref_body(uint32_t bx, const float2* __restrict__ pos,
+// 1 / sqrt(x) with both operations correctly rounded, for two values at once: the value of
+// __frcp_rn(__fsqrt_rn(x)).  The method is Markstein's (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): from
+// an approximation y of 1/sqrt(x), a Newton step in g ~ sqrt(x) and h ~ 1/(2 sqrt(x))
+//     g = x y, h = y / 2, e = 1/2 - g h, g += g e, h += h e,
+// then the residual x - g^2, exact in an FMA, gives the rounded root s = g + (x - g^2) h, and two
+// steps r += (1 - s r) r from r = 2 h the rounded reciprocal (one leaves two mantissas, whose
+// reciprocals lie 5e-8 of a unit from a rounding boundary, one unit off).  No step overflows
+// or loses bits to underflow for x in [2^-100, 2^100].  A root of all-ones mantissa, the case
+// Markstein's theorem on reciprocals leaves out, comes from an x of all-ones mantissa.  Those,
+// and an x outside the range (a zero, a NaN, an overflowed distance), go to the library
+// functions; compared with them on the GPU, every float from 0 to infinity is equal.  In packed f32x2
+// form the chain is 6.5 issues a value; the library's root and reciprocal carry their own
+// range checks and branches, most of the 47 instructions that a factor cost.
+__device__ __forceinline__ float2 ref_inv_sqrt2(float2 x) {
+    const float2 y = make_float2(direct_rsqrt<true>(x.x), direct_rsqrt<true>(x.y));
+    float2 g = mul2(x, y), h = mul2(y, make_float2(0.5f, 0.5f));
+    const float2 e = fma2(make_float2(-g.x, -g.y), h, make_float2(0.5f, 0.5f));
+    g = fma2(g, e, g);
+    h = fma2(h, e, h);
+    const float2 s = fma2(fma2(make_float2(-g.x, -g.y), g, x), h, g);
+    const float2 ns = make_float2(-s.x, -s.y), one = make_float2(1.0f, 1.0f);
+    const float2 r = add2(h, h), r1 = fma2(fma2(ns, r, one), r, r);
+    float2 v = fma2(fma2(ns, r1, one), r1, r1);
+    const float lo = 7.888609052e-31f, hi = 1.267650600e30f;  // 2^-100, 2^100
+    const uint32_t ones = 0x7fffffu;
+    if (!(x.x >= lo && x.x <= hi && x.y >= lo && x.y <= hi) || (__float_as_uint(x.x) & ones) == ones ||
+        (__float_as_uint(x.y) & ones) == ones) {
+        v.x = __frcp_rn(__fsqrt_rn(x.x));
+        v.y = __frcp_rn(__fsqrt_rn(x.y));
+    }
+    return v;
+}
+
+// REFERENCE math: 32 targets per block.  The shader's sum takes the sources in order
+// (SimShader.comp:43-65), but only the two additions of each pair depend on the pair before;
+// the factors s = ((m r) r) r with r = 1 / sqrt(d2), both correctly rounded, do not.  So 16
+// warps make the factors of a 64-source tile (lane: target, four sources per warp, two per
+// packed instruction) in shared memory while two more add up an earlier tile, one the x and
+// one the y sums, each lane its own target in source order.  One thread per particle doing
+// both was bound by its own chain of dependent divisions (N = 4096: 128 warps on the whole
+// chip, 328 us a step).
+constexpr int kRefWarps = 16;                        // warps that make factors
+constexpr int kRefThreads = (kRefWarps + 2) * 32;
+constexpr uint32_t kRefTargets = 32;
+constexpr int kRefPer = 4;                           // sources per warp and tile: two float4 of positions, one of masses
+constexpr int kRefTile = kRefWarps * kRefPer;
+static_assert(kAlignment % kRefTile == 0, "whole tiles");
+
+// Tiles of factors in flight between the making and the adding warps.
+constexpr int kRefRing = 4;
+
+struct DirectRefSmem {
+    float s[kRefRing][kRefTile][kRefTargets];
+    float c[kRefRing][2][kRefTile];  // the tile's x and y
+    float a[kRefTargets];
+};
+
+// Named barriers of ring slot b: full (1 + b), its factors are made; empty (1 + kRefRing + b),
+// they have been added up.  Both count every thread of the block: one side arrives, the other
+// waits.
+__device__ __forceinline__ void ref_arrive(uint32_t id) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kRefThreads) : "memory");
+}
+__device__ __forceinline__ void ref_wait(uint32_t id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kRefThreads) : "memory");
+}
+
+// The factors of two sources for one target: dx, dy, d2 = fma(dx, dx, fma(dy, dy, eps2)), then
+// ((m r) r) r, each lane rounding like the scalar operations.
+__device__ __forceinline__ float2 ref_factors(float2 x, float2 y, float2 m, float2 P, float2 Q, float2 E2) {
+    const float2 dx = sub2(x, P), dy = sub2(y, Q);
+    const float2 r = ref_inv_sqrt2(fma2(dx, dx, fma2(dy, dy, E2)));
+    return mul2(mul2(mul2(m, r), r), r);
+}
+
+__device__ __forceinline__ void direct_ref_body(DirectRefSmem& g, uint32_t bx, const float2* __restrict__ pos,
                                                 const float2* __restrict__ vel, const float* __restrict__ mass,
                                                 float2* __restrict__ pos_out, float2* __restrict__ vel_out,
                                                 float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float k,
                                                 float hdt) {
-    __shared__ float2 sp[64];
-    __shared__ float sm[64];
-    const uint32_t i = bx * 64 + threadIdx.x;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t i = bx * kRefTargets + lane, tiles = n_al / kRefTile;
     const float2 p = pos[i];
-    float ax = 0.f, ay = 0.f;
-    for (uint32_t jt = 0; jt < n_al; jt += 64) {  // SimShader.comp:43-65
-        sp[threadIdx.x] = pos[jt + threadIdx.x];
-        sm[threadIdx.x] = mass[jt + threadIdx.x];
-        __syncthreads();
-        for (int jj = 0; jj < 64; ++jj) {
-            float dx = sp[jj].x - p.x;
-            float dy = sp[jj].y - p.y;
-            float d2 = fmaf(dx, dx, fmaf(dy, dy, eps2));
-            float r = __fdiv_rn(1.0f, __fsqrt_rn(d2));
-            float s = ((sm[jj] * r) * r) * r;
-            ax = fmaf(dx, s, ax);
-            ay = fmaf(dy, s, ay);
-        }
-        __syncthreads();
+    const float2 P = make_float2(p.x, p.x), Q = make_float2(p.y, p.y), E2 = make_float2(eps2, eps2);
+    const float4* pos2 = reinterpret_cast<const float4*>(pos);
+    const float4* mass4 = reinterpret_cast<const float4*>(mass);
+    const int f = w * kRefPer;  // the warp's first source of a tile
+    // the sources of this tile and of the next two: a tile is made in less than an L2 round trip
+    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, m = q0, q0b = q0, q1b = q0, mb = q0;
+    const auto load = [&](uint32_t jt, float4& a0, float4& a1, float4& am) {
+        const uint32_t n0 = jt * kRefTile + f;
+        a0 = __ldg(&pos2[n0 / 2]);
+        a1 = __ldg(&pos2[n0 / 2 + 1]);
+        am = __ldg(&mass4[n0 / 4]);
+    };
+    if (w < kRefWarps) {
+        load(0, q0, q1, m);
+        if (tiles > 1) load(1, q0b, q1b, mb);
     }
+    const int axis = w - kRefWarps;  // of an adding warp: 0 x, 1 y
+    const float pc = axis ? p.y : p.x;
+    float a = 0.f;
+    if (w < kRefWarps) {
+        for (uint32_t jt = 0; jt < tiles; ++jt) {
+            const uint32_t b = jt % kRefRing;
+            const float4 p0 = q0, p1 = q1, pm = m;
+            q0 = q0b;
+            q1 = q1b;
+            m = mb;
+            if (jt + 2 < tiles) load(jt + 2, q0b, q1b, mb);
+            const float2 sa = ref_factors(make_float2(p0.x, p0.z), make_float2(p0.y, p0.w), make_float2(pm.x, pm.y), P,
+                                          Q, E2);
+            const float2 sb = ref_factors(make_float2(p1.x, p1.z), make_float2(p1.y, p1.w), make_float2(pm.z, pm.w), P,
+                                          Q, E2);
+            if (jt >= kRefRing) ref_wait(1 + kRefRing + b);
+            g.s[b][f][lane] = sa.x;
+            g.s[b][f + 1][lane] = sa.y;
+            g.s[b][f + 2][lane] = sb.x;
+            g.s[b][f + 3][lane] = sb.y;
+            if (lane < kRefPer) {
+                g.c[b][0][f + lane] = lane == 0 ? p0.x : lane == 1 ? p0.z : lane == 2 ? p1.x : p1.z;
+                g.c[b][1][f + lane] = lane == 0 ? p0.y : lane == 1 ? p0.w : lane == 2 ? p1.y : p1.w;
+            }
+            ref_arrive(1 + b);
+        }
+    } else {
+        for (uint32_t jt = 0; jt < tiles; ++jt) {
+            const uint32_t b = jt % kRefRing;
+            ref_wait(1 + b);
+            // eight sources at a time, the next eight's factors and coordinates loaded before
+            // the sums of this eight: the chain of dependent additions is the block's pace
+            const float4* c4 = reinterpret_cast<const float4*>(g.c[b][axis]);
+            float sv[8], sn[8];
+            float4 c0 = c4[0], c1 = c4[1], n0 = c0, n1 = c1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) sv[u] = g.s[b][u][lane];
+#pragma unroll
+            for (int t = 0; t < kRefTile; t += 8) {
+                if (t + 8 < kRefTile) {
+                    n0 = c4[t / 4 + 2];
+                    n1 = c4[t / 4 + 3];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) sn[u] = g.s[b][t + 8 + u][lane];
+                }
+                const float d[8] = {c0.x - pc, c0.y - pc, c0.z - pc, c0.w - pc, c1.x - pc, c1.y - pc, c1.z - pc, c1.w - pc};
+#pragma unroll
+                for (int u = 0; u < 8; ++u) a = fmaf(d[u], sv[u], a);
+                c0 = n0;
+                c1 = n1;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) sv[u] = sn[u];
+            }
+            if (jt + kRefRing < tiles) ref_arrive(1 + kRefRing + b);  // one for each later wait
+        }
+    }
+    if (axis == 1) g.a[lane] = a;
+    __syncthreads();
+    if (axis != 0) return;
+    const float ax = a, ay = g.a[lane];
     if (acc_rec) acc_rec[i] = make_float2(ax, ay);
-    float2 v = vel[i];
-    float nvx = fmaf(ax, k, v.x), nvy = fmaf(ay, k, v.y);
+    const float2 v = vel[i];
+    const float nvx = fmaf(ax, k, v.x), nvy = fmaf(ay, k, v.y);
     pos_out[i] = make_float2(fmaf(v.x + nvx, hdt, p.x), fmaf(v.y + nvy, hdt, p.y));
     vel_out[i] = make_float2(nvx, nvy);
 }
@@ -372,12 +507,13 @@ k_direct_fast(const float2* __restrict__ pos, const float2* __restrict__ vel, co
                                       jchunk, eps2, k, hdt, partials, tickets);
 }
 
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(kRefThreads, 2)
 k_direct_ref(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
              float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
              uint32_t n_al, float eps2, float k, float hdt) {
     chain_enter();
-    direct_ref_body(blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
+    __shared__ __align__(16) DirectRefSmem g;
+    direct_ref_body(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
 }
 
 // Batched direct sum: one launch over every direct-sum system of a plan.  Block b belongs
@@ -407,14 +543,15 @@ __device__ __forceinline__ void direct_batch_body(DirectSmallSmem<kDirectBlock /
 }
 
 template <bool EXACT, bool KAHAN, int IPT>
-__global__ void __launch_bounds__(EXACT ? 64 : kDirectBlock, IPT == 4 ? 6 : 8)
+__global__ void __launch_bounds__(EXACT ? kRefThreads : kDirectBlock, EXACT ? 2 : IPT == 4 ? 6 : 8)
 kb_direct(const SysDesc* __restrict__ descs, const uint32_t* __restrict__ first, uint32_t nsys, uint32_t step) {
     const uint32_t s = direct_batch_sys(first, nsys, blockIdx.x);
     const SysDesc& d = descs[s];
     const uint32_t b = blockIdx.x - __ldg(&first[s]);
     const int in = (int)((d.parity + step) & 1u), out = in ^ 1;
     if constexpr (EXACT) {
-        direct_ref_body(b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.k,
+        __shared__ __align__(16) DirectRefSmem g;
+        direct_ref_body(g, b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.k,
                         d.hdt);
     } else {
         __shared__ __align__(16) DirectSmallSmem<kDirectBlock / 32> g;
@@ -626,7 +763,7 @@ cudaError_t direct_step(gs_sim* s, int in, int out, bool profile, bool chained) 
     cudaError_t e;
     stage_begin(s, kStageDirect, profile);
     if (s->p.math_mode == GS_MATH_REFERENCE)
-        e = launch(pdl, k_direct_ref, dim3(n_al / 64), 64, s->stream, s->pos[in], s->vel[in],
+        e = launch(pdl, k_direct_ref, dim3(n_al / kRefTargets), kRefThreads, s->stream, s->pos[in], s->vel[in],
                    s->mass[in], s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k, hdt);
     else
         e = direct_fast_launch(pdl, direct_grid(s), shape_ipt(s->shape), (s->p.flags & GS_FLAG_PLAIN_SUM) != 0,
@@ -645,7 +782,7 @@ void direct_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const 
     d.jchunk = g.jchunk;
     d.partials = s->dw.partials;
     d.tickets = s->dw.tickets;
-    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? (uint32_t)(s->n_al / 64)
+    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? (uint32_t)(s->n_al / kRefTargets)
                          : g.chunks                          ? d.itiles * g.chunks
                                                              : (uint32_t)(s->n_al / 32);
 }
@@ -655,7 +792,7 @@ cudaError_t direct_batch_step(const BatchPlan& p, uint32_t step, cudaStream_t st
     const SysDesc* descs = p.d_descs + p.n_bh;
     const bool four = shape_ipt(p.shape) == 4;
     if (p.direct_exact)
-        kb_direct<true, false, 2><<<p.total[kTabDirect], 64, 0, st>>>(descs, p.d_tab[kTabDirect], p.n_direct, step);
+        kb_direct<true, false, 2><<<p.total[kTabDirect], kRefThreads, 0, st>>>(descs, p.d_tab[kTabDirect], p.n_direct, step);
     else
         (p.direct_plain ? (four ? kb_direct<false, false, 4> : kb_direct<false, false, 2>)
                         : (four ? kb_direct<false, true, 4> : kb_direct<false, true, 2>))
