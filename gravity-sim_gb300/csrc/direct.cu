@@ -399,8 +399,10 @@ __device__ __forceinline__ void ref_wait(uint32_t id) {
 
 // The factors of two sources for one target: dx, dy, d2 = fma(dx, dx, fma(dy, dy, eps2)), then
 // ((m r) r) r, each lane rounding like the scalar operations.
-__device__ __forceinline__ float2 ref_factors(float2 x, float2 y, float2 m, float2 P, float2 Q, float2 E2) {
-    const float2 dx = sub2(x, P), dy = sub2(y, Q);
+__device__ __forceinline__ float2 ref_factors(float2 x, float2 y, float2 m, float2 P, float2 Q, float2 E2, float2& dx,
+                                              float2& dy) {
+    dx = sub2(x, P);
+    dy = sub2(y, Q);
     const float2 r = ref_inv_sqrt2(fma2(dx, dx, fma2(dy, dy, E2)));
     return mul2(mul2(mul2(m, r), r), r);
 }
@@ -440,10 +442,11 @@ __device__ __forceinline__ void direct_ref_body(DirectRefSmem& g, uint32_t bx, c
             q1 = q1b;
             m = mb;
             if (jt + 2 < tiles) load(jt + 2, q0b, q1b, mb);
+            float2 dx, dy;
             const float2 sa = ref_factors(make_float2(p0.x, p0.z), make_float2(p0.y, p0.w), make_float2(pm.x, pm.y), P,
-                                          Q, E2);
+                                          Q, E2, dx, dy);
             const float2 sb = ref_factors(make_float2(p1.x, p1.z), make_float2(p1.y, p1.w), make_float2(pm.z, pm.w), P,
-                                          Q, E2);
+                                          Q, E2, dx, dy);
             if (jt >= kRefRing) ref_wait(1 + kRefRing + b);
             g.s[b][f][lane] = sa.x;
             g.s[b][f + 1][lane] = sa.y;
@@ -494,6 +497,85 @@ __device__ __forceinline__ void direct_ref_body(DirectRefSmem& g, uint32_t bx, c
     const float nvx = fmaf(ax, k, v.x), nvy = fmaf(ay, k, v.y);
     pos_out[i] = make_float2(fmaf(v.x + nvx, hdt, p.x), fmaf(v.y + nvy, hdt, p.y));
     vel_out[i] = make_float2(nvx, nvy);
+}
+
+// REFERENCE math, large systems: a warp per 32 targets makes the factors and adds them up
+// itself, four sources at a time.  There are warps enough to hide each one's chain, and
+// nothing is handed over.
+template <int W>
+struct DirectRowsSmem {
+    float x[W][kDirectTileJ], y[W][kDirectTileJ], m[W][kDirectTileJ];
+};
+constexpr int kRowsWarps = 2;
+
+template <int W>
+__device__ __forceinline__ void direct_rows_body(DirectRowsSmem<W>& g, uint32_t bx, const float2* __restrict__ pos,
+                                                 const float2* __restrict__ vel, const float* __restrict__ mass,
+                                                 float2* __restrict__ pos_out, float2* __restrict__ vel_out,
+                                                 float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float k,
+                                                 float hdt) {
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t i = (bx * W + w) * 32 + lane, tiles = n_al / kDirectTileJ;
+    if (i >= n_al) return;  // the whole warp: n_al is a multiple of 64
+    const float2 p = pos[i];
+    const float2 P = make_float2(p.x, p.x), Q = make_float2(p.y, p.y), E2 = make_float2(eps2, eps2);
+    const float4* X = reinterpret_cast<const float4*>(g.x[w]);
+    const float4* Y = reinterpret_cast<const float4*>(g.y[w]);
+    const float4* M = reinterpret_cast<const float4*>(g.m[w]);
+    float ax = 0.f, ay = 0.f;
+    float4 q = reinterpret_cast<const float4*>(pos)[lane];  // two positions and their masses
+    float2 m = reinterpret_cast<const float2*>(mass)[lane];
+    for (uint32_t jt = 0; jt < tiles; ++jt) {
+        __syncwarp();
+        reinterpret_cast<float2*>(g.x[w])[lane] = make_float2(q.x, q.z);
+        reinterpret_cast<float2*>(g.y[w])[lane] = make_float2(q.y, q.w);
+        reinterpret_cast<float2*>(g.m[w])[lane] = m;
+        __syncwarp();
+        if (jt + 1 < tiles) {  // in flight while this tile is summed
+            q = reinterpret_cast<const float4*>(pos)[(jt + 1) * 32 + lane];
+            m = reinterpret_cast<const float2*>(mass)[(jt + 1) * 32 + lane];
+        }
+#pragma unroll 2
+        for (int jj = 0; jj < kDirectTileJ / 4; ++jj) {
+            const float4 x = X[jj], y = Y[jj], c = M[jj];
+            float2 dxa, dya, dxb, dyb;
+            const float2 sa = ref_factors(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(c.x, c.y), P, Q, E2,
+                                          dxa, dya);
+            const float2 sb = ref_factors(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(c.z, c.w), P, Q, E2,
+                                          dxb, dyb);
+            ax = fmaf(dxa.x, sa.x, ax);
+            ay = fmaf(dya.x, sa.x, ay);
+            ax = fmaf(dxa.y, sa.y, ax);
+            ay = fmaf(dya.y, sa.y, ay);
+            ax = fmaf(dxb.x, sb.x, ax);
+            ay = fmaf(dyb.x, sb.x, ay);
+            ax = fmaf(dxb.y, sb.y, ax);
+            ay = fmaf(dyb.y, sb.y, ay);
+        }
+    }
+    if (acc_rec) acc_rec[i] = make_float2(ax, ay);
+    const float2 v = vel[i];
+    const float nvx = fmaf(ax, k, v.x), nvy = fmaf(ay, k, v.y);
+    pos_out[i] = make_float2(fmaf(v.x + nvx, hdt, p.x), fmaf(v.y + nvy, hdt, p.y));
+    vel_out[i] = make_float2(nvx, nvy);
+}
+
+// Which REFERENCE-math kernel a system takes (the same bits either way), and its blocks.
+// N = 12,288: 316 us a step on k_direct_ref, 409 here; 16,384: 548 and 543; 50,000: 4464 and 2486
+// (4330 with a thread per particle and the library's root and division).
+constexpr uint32_t kRefSplitMax = 16384;
+__host__ __device__ __forceinline__ bool ref_rows(uint32_t n_al) { return n_al > kRefSplitMax; }
+static uint32_t ref_blocks(uint32_t n_al, int rows_warps) {
+    return ref_rows(n_al) ? (n_al / 32 + rows_warps - 1) / rows_warps : n_al / kRefTargets;
+}
+
+__global__ void __launch_bounds__(kRowsWarps * 32)
+k_direct_rows(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
+              float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec, uint32_t n_al,
+              float eps2, float k, float hdt) {
+    chain_enter();
+    __shared__ __align__(16) DirectRowsSmem<kRowsWarps> g;
+    direct_rows_body<kRowsWarps>(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
 }
 
 template <int IPT, bool KAHAN, bool FTZ>
@@ -550,9 +632,16 @@ kb_direct(const SysDesc* __restrict__ descs, const uint32_t* __restrict__ first,
     const uint32_t b = blockIdx.x - __ldg(&first[s]);
     const int in = (int)((d.parity + step) & 1u), out = in ^ 1;
     if constexpr (EXACT) {
-        __shared__ __align__(16) DirectRefSmem g;
-        direct_ref_body(g, b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.k,
-                        d.hdt);
+        __shared__ __align__(16) union {
+            DirectRefSmem split;
+            DirectRowsSmem<kRefThreads / 32> rows;
+        } g;
+        if (ref_rows(d.n_al))
+            direct_rows_body<kRefThreads / 32>(g.rows, b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out],
+                                               d.acc, d.n_al, d.eps2, d.k, d.hdt);
+        else
+            direct_ref_body(g.split, b, d.pos[in], d.vel[in], d.mass[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2,
+                            d.k, d.hdt);
     } else {
         __shared__ __align__(16) DirectSmallSmem<kDirectBlock / 32> g;
         if (direct_ftz(d.eps2)) direct_batch_body<IPT, KAHAN, true>(g, d, b, in, out);
@@ -763,8 +852,9 @@ cudaError_t direct_step(gs_sim* s, int in, int out, bool profile, bool chained) 
     cudaError_t e;
     stage_begin(s, kStageDirect, profile);
     if (s->p.math_mode == GS_MATH_REFERENCE)
-        e = launch(pdl, k_direct_ref, dim3(n_al / kRefTargets), kRefThreads, s->stream, s->pos[in], s->vel[in],
-                   s->mass[in], s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k, hdt);
+        e = launch(pdl, ref_rows(n_al) ? k_direct_rows : k_direct_ref, dim3(ref_blocks(n_al, kRowsWarps)),
+                   ref_rows(n_al) ? kRowsWarps * 32 : kRefThreads, s->stream, s->pos[in], s->vel[in], s->mass[in],
+                   s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k, hdt);
     else
         e = direct_fast_launch(pdl, direct_grid(s), shape_ipt(s->shape), (s->p.flags & GS_FLAG_PLAIN_SUM) != 0,
                                s->pos[in], s->vel[in], s->mass[in], s->pos[out], s->vel[out], s->acc, n_al, s->eps2, k,
@@ -782,7 +872,7 @@ void direct_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const 
     d.jchunk = g.jchunk;
     d.partials = s->dw.partials;
     d.tickets = s->dw.tickets;
-    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? (uint32_t)(s->n_al / kRefTargets)
+    blocks[kTabDirect] = s->p.math_mode == GS_MATH_REFERENCE ? ref_blocks((uint32_t)s->n_al, kRefThreads / 32)
                          : g.chunks                          ? d.itiles * g.chunks
                                                              : (uint32_t)(s->n_al / 32);
 }

@@ -48,7 +48,7 @@ def test_fast_subnormal_softening(gs, orc, n):
     assert _rms(acc[t], a64) < 2e-6
 
 
-@pytest.mark.parametrize("n", [64, 4160])
+@pytest.mark.parametrize("n", [64, 4160, 16448])
 @pytest.mark.parametrize("scale,mass_scale,softening", [(1.0, 1.0, 0.2), (1e13, 1.0, 0.2), (1e17, 1.0, 0.2),
                                                         (1e19, 1.0, 0.2), (1e-17, 1e-25, 1e-19)])
 def test_reference_ranges_bit_exact(gs, orc, n, scale, mass_scale, softening):
