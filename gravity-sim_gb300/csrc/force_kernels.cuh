@@ -3,6 +3,8 @@
 // templated on the math mode and on the launch shape (gs_shape: warps per block, list
 // caps).  force_fast.cu and force_exact.cu instantiate them for FAST and REFERENCE math.
 #pragma once
+#include <type_traits>
+
 #include "bh_common.cuh"
 
 namespace gsim {
@@ -12,18 +14,52 @@ namespace {
 // traversal + integrator (ForceShader.comp:78-152)
 // ------------------------------------------------------------------------------------
 
-template <bool EXACT, bool COUNT>
-__device__ __forceinline__ void force_body(Blk blk, const uint32_t* __restrict__ sidx,
-                                           const uint32_t* __restrict__ counts, const float4* __restrict__ rec,
-                                           const uint32_t* __restrict__ skip, const float2* __restrict__ pos_in,
-                                           const float2* __restrict__ vel_in, float2* __restrict__ pos_out,
-                                           float2* __restrict__ vel_out, float2* __restrict__ acc_rec, uint32_t n_al,
-                                           float eps2, float theta2, float k, float hdt, uint32_t cap,
-                                           unsigned long long* __restrict__ stat, uint32_t* __restrict__ ext) {
-    __shared__ float4 wrec[kForceWarps][32];
-    __shared__ uint32_t wskip[kForceWarps][32];
+// 1/sqrt: correctly rounded (REFERENCE math) or the hardware approximation (FAST math;
+// d2 >= eps^2 > 0 is never subnormal, so the flush-to-zero form loses nothing)
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+template <bool EXACT>
+__device__ __forceinline__ float inv_sqrt(float d2) {
+    return EXACT ? __fdiv_rn(1.0f, __fsqrt_rn(d2)) : rsqrt_fast(d2);
+}
+
+// FAST math of the reference rule, whose softening may be so small that d2 is subnormal
+// (FTZ false: the form that scales such inputs); with a normal eps^2 both give the same bits.
+template <bool EXACT, bool FTZ>
+__device__ __forceinline__ float rule_inv_sqrt(float d2) {
+    if (EXACT) return __fdiv_rn(1.0f, __fsqrt_rn(d2));
+    return FTZ ? rsqrt_fast(d2) : rsqrtf(d2);
+}
+__host__ __device__ __forceinline__ bool rule_ftz(float eps2) { return eps2 >= 1.17549435e-38f; }
+
+// Shared memory of a warp's walk: a window of 32 records from `base` on.
+struct RuleWindow {
+    float4 rec[32];
+    uint32_t skip[32];
+};
+
+// A warp's walk of the preorder records.  Records are taken four at a time: their distances
+// and tests are made together (two records per packed instruction), and when all four are
+// accepted and follow one another (particle leaves) all four are summed at once; otherwise
+// the four are gone through in order with the distances at hand, as the rule does one by
+// one.  The sums take the records in the same order either way.
+// win: the warp's window, or with STAGED (win unused) the whole tree in shared memory at
+// s_rec / s_skip.
+template <bool EXACT, bool COUNT, bool FTZ, bool STAGED>
+__device__ __forceinline__ void force_body(Blk blk, RuleWindow* win, const float4* s_rec, const uint32_t* s_skip,
+                                           const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ counts,
+                                           const float4* __restrict__ rec, const uint32_t* __restrict__ skip,
+                                           const float2* __restrict__ pos_in, const float2* __restrict__ vel_in,
+                                           float2* __restrict__ pos_out, float2* __restrict__ vel_out,
+                                           float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float theta2,
+                                           float k, float hdt, uint32_t cap, unsigned long long* __restrict__ stat,
+                                           uint32_t* __restrict__ ext) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t group = blk.id * kForceWarps + warp;
+    const uint32_t group = blk.id * (blockDim.x >> 5) + warp;
     const uint32_t nv = counts[0];
     const uint32_t T = min(nv + counts[1], cap);  // preorder records
     if (group * 32 >= nv) return;       // no particle in this warp: nothing to write
@@ -31,35 +67,75 @@ __device__ __forceinline__ void force_body(Blk blk, const uint32_t* __restrict__
     const uint32_t i = s < nv ? sidx[s] : 0u;
     const bool valid = s < nv && i < n_al;  // i < n_al unless the sort failed (error flag set)
     const float2 p = valid ? pos_in[i] : make_float2(0.0f, 0.0f);
+    const float2 P = make_float2(p.x, p.x), Q = make_float2(p.y, p.y), E2 = make_float2(eps2, eps2);
+    const float2 TH = make_float2(theta2, theta2);
     float ax = 0.0f, ay = 0.0f;
     unsigned long long n_acc = 0, n_vis = 0;
     uint32_t base = 0, ind = 0;
-    wrec[warp][lane] = rec[lane];
-    wskip[warp][lane] = skip[lane];
-    __syncwarp();
+    if (!STAGED) {
+        win->rec[lane] = rec[lane];
+        win->skip[lane] = skip[lane];
+        __syncwarp();
+    }
     while (ind < T) {
-        if (ind - base >= 32u) {  // warp-uniform: reload the 32-record window
-            base = ind & ~31u;
+        if (!STAGED && ind - base > 28u) {  // warp-uniform: fewer than four records left in the window
+            base = ind;
             __syncwarp();
-            wrec[warp][lane] = rec[base + lane];
-            wskip[warp][lane] = skip[base + lane];
+            win->rec[lane] = rec[base + lane];  // the arrays end 32 records past cap
+            win->skip[lane] = skip[base + lane];
             __syncwarp();
         }
-        const float4 q = wrec[warp][ind - base];
-        const float dx = q.x - p.x, dy = q.y - p.y;
-        const float d2 = fmaf(dx, dx, fmaf(dy, dy, eps2));
-        const bool ok = !valid || q.w <= d2 * theta2;
-        if (COUNT) ++n_vis;
-        if (__all_sync(0xffffffffu, ok)) {
-            const float r = EXACT ? __fdiv_rn(1.0f, __fsqrt_rn(d2)) : rsqrtf(d2);
-            const float sc = ((q.z * r) * r) * r;
-            ax = fmaf(dx, sc, ax);
-            ay = fmaf(dy, sc, ay);
-            if (COUNT) n_acc += valid;
-            ind += max(wskip[warp][ind - base], 1u);  // >= 1: the walk always advances
-        } else {
-            ++ind;
+        const float4* q = STAGED ? s_rec + ind : win->rec + (ind - base);
+        const uint32_t* sk = STAGED ? s_skip + ind : win->skip + (ind - base);
+        const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3];
+        const float2 dxa = sub2(make_float2(q0.x, q1.x), P), dya = sub2(make_float2(q0.y, q1.y), Q);
+        const float2 dxb = sub2(make_float2(q2.x, q3.x), P), dyb = sub2(make_float2(q2.y, q3.y), Q);
+        const float2 da = fma2(dxa, dxa, fma2(dya, dya, E2)), db = fma2(dxb, dxb, fma2(dyb, dyb, E2));
+        const float2 ta = mul2(da, TH), tb = mul2(db, TH);
+        const bool ok[4] = {!valid || q0.w <= ta.x, !valid || q1.w <= ta.y, !valid || q2.w <= tb.x,
+                            !valid || q3.w <= tb.y};
+        const uint32_t sk0 = sk[0], sk1 = sk[1], sk2 = sk[2], sk3 = sk[3];
+        const uint32_t left = T - ind;
+        if (left >= 4u && (sk0 | sk1 | sk2) == 1u && __all_sync(0xffffffffu, ok[0] && ok[1] && ok[2] && ok[3])) {
+            const float2 ra = make_float2(rule_inv_sqrt<EXACT, FTZ>(da.x), rule_inv_sqrt<EXACT, FTZ>(da.y));
+            const float2 rb = make_float2(rule_inv_sqrt<EXACT, FTZ>(db.x), rule_inv_sqrt<EXACT, FTZ>(db.y));
+            const float2 sa = mul2(mul2(mul2(make_float2(q0.z, q1.z), ra), ra), ra);
+            const float2 sb = mul2(mul2(mul2(make_float2(q2.z, q3.z), rb), rb), rb);
+            ax = fmaf(dxa.x, sa.x, ax);
+            ay = fmaf(dya.x, sa.x, ay);
+            ax = fmaf(dxa.y, sa.y, ax);
+            ay = fmaf(dya.y, sa.y, ay);
+            ax = fmaf(dxb.x, sb.x, ax);
+            ay = fmaf(dyb.x, sb.x, ay);
+            ax = fmaf(dxb.y, sb.y, ax);
+            ay = fmaf(dyb.y, sb.y, ay);
+            if (COUNT) {
+                n_vis += 4;
+                n_acc += valid ? 4 : 0;
+            }
+            ind += 3u + max(sk3, 1u);  // >= 1: the walk always advances
+            continue;
         }
+        const float qm[4] = {q0.z, q1.z, q2.z, q3.z}, dd[4] = {da.x, da.y, db.x, db.y};
+        const float dx[4] = {dxa.x, dxa.y, dxb.x, dxb.y}, dy[4] = {dya.x, dya.y, dyb.x, dyb.y};
+        const uint32_t sks[4] = {sk0, sk1, sk2, sk3};
+        uint32_t next = 0;  // the next record of the rule's walk, from ind
+#pragma unroll
+        for (uint32_t t = 0; t < 4; ++t) {
+            if (next != t || t >= left) continue;  // uniform
+            if (COUNT) ++n_vis;
+            if (__all_sync(0xffffffffu, ok[t])) {
+                const float r = rule_inv_sqrt<EXACT, FTZ>(dd[t]);
+                const float sc = ((qm[t] * r) * r) * r;
+                ax = fmaf(dx[t], sc, ax);
+                ay = fmaf(dy[t], sc, ay);
+                if (COUNT) n_acc += valid;
+                next += max(sks[t], 1u);
+            } else {
+                ++next;
+            }
+        }
+        ind += next;
     }
     if (COUNT) {
         for (int o = 16; o; o >>= 1) n_acc += __shfl_xor_sync(0xffffffffu, n_acc, o);
@@ -82,16 +158,63 @@ __device__ __forceinline__ void force_body(Blk blk, const uint32_t* __restrict__
                 valid ? np.y : -INFINITY);
 }
 
-template <bool EXACT, bool COUNT>
+template <bool EXACT, bool COUNT, bool FTZ>
 __global__ void __launch_bounds__(kForceWarps * 32)
 k_force(const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ counts, const float4* __restrict__ rec,
         const uint32_t* __restrict__ skip, const float2* __restrict__ pos_in, const float2* __restrict__ vel_in,
         float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec, uint32_t n_al,
         float eps2, float theta2, float k, float hdt, uint32_t cap, unsigned long long* __restrict__ stat,
         uint32_t* __restrict__ ext) {
+    __shared__ RuleWindow win[kForceWarps];
     pdl_enter();
-    force_body<EXACT, COUNT>(grid_blk(), sidx, counts, rec, skip, pos_in, vel_in, pos_out, vel_out, acc_rec, n_al,
-                             eps2, theta2, k, hdt, cap, stat, ext);
+    force_body<EXACT, COUNT, FTZ, false>(grid_blk(), &win[threadIdx.x >> 5], nullptr, nullptr, sidx, counts, rec, skip,
+                                         pos_in, vel_in, pos_out, vel_out, acc_rec, n_al, eps2, theta2, k, hdt, cap,
+                                         stat, ext);
+}
+
+// Small systems: fewer blocks than SMs, so every walk's latency counts, and a window reload
+// per accepted node is an L2 round trip (N = 3000: 36 us for some 150 visits a warp).  Each
+// block first copies the whole tree into its shared memory; a tree that does not fit
+// (kRuleStage records) is walked through windows as above.
+constexpr uint32_t kRuleStage = 10240;           // records: 200 KB of records and skips
+constexpr uint32_t kRuleStagedMax = 1u << 13;    // particles; one block per SM at most
+struct RuleTree {
+    float4 rec[kRuleStage + 8];
+    uint32_t skip[kRuleStage + 8];
+};
+
+template <bool EXACT, bool COUNT, bool FTZ>
+__global__ void __launch_bounds__(kForceWarps * 32)
+k_force_staged(const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ counts, const float4* __restrict__ rec,
+               const uint32_t* __restrict__ skip, const float2* __restrict__ pos_in,
+               const float2* __restrict__ vel_in, float2* __restrict__ pos_out, float2* __restrict__ vel_out,
+               float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float theta2, float k, float hdt, uint32_t cap,
+               unsigned long long* __restrict__ stat, uint32_t* __restrict__ ext) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    RuleTree& tree = *reinterpret_cast<RuleTree*>(s_raw);
+    pdl_enter();
+    const uint32_t T = min(counts[0] + counts[1], cap);
+    if (T > kRuleStage) {
+        force_body<EXACT, COUNT, FTZ, false>(grid_blk(), reinterpret_cast<RuleWindow*>(s_raw) + (threadIdx.x >> 5),
+                                             nullptr, nullptr, sidx, counts, rec, skip, pos_in, vel_in, pos_out,
+                                             vel_out, acc_rec, n_al, eps2, theta2, k, hdt, cap, stat, ext);
+        return;
+    }
+    // the last four-record round reads up to three records past the end (the arrays hold
+    // cap + 32); they never enter a sum
+    const uint32_t rows = (T + 3 + 3) & ~3u;
+    for (uint32_t r = threadIdx.x; r < rows; r += kForceWarps * 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&tree.rec[r])),
+                     "l"(rec + r)
+                     : "memory");
+    for (uint32_t r = 4 * threadIdx.x; r < rows; r += 4 * kForceWarps * 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&tree.skip[r])),
+                     "l"(skip + r)
+                     : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    force_body<EXACT, COUNT, FTZ, true>(grid_blk(), nullptr, tree.rec, tree.skip, sidx, counts, rec, skip, pos_in,
+                                        vel_in, pos_out, vel_out, acc_rec, n_al, eps2, theta2, k, hdt, cap, stat, ext);
 }
 
 // ------------------------------------------------------------------------------------
@@ -110,19 +233,6 @@ static_assert(kStackCap >= 96 * (kBBoxMaxBits > kFixedDepth ? kBBoxMaxBits : kFi
 // Accepted nodes and runs of particle leaves collected between evaluations: 160 / 128
 // (long lists) or 96 / 64 (short lists, gs_shape.force_short_lists); a pop adds at most
 // 32 nodes and 64 runs.
-
-// 1/sqrt: correctly rounded (REFERENCE math) or the hardware approximation (FAST math;
-// d2 >= eps^2 > 0 is never subnormal, so the flush-to-zero form loses nothing)
-__device__ __forceinline__ float rsqrt_fast(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-template <bool EXACT>
-__device__ __forceinline__ float inv_sqrt(float d2) {
-    return EXACT ? __fdiv_rn(1.0f, __fsqrt_rn(d2)) : rsqrt_fast(d2);
-}
 
 // Evaluation order.  Each particle sums the accepted nodes and the particle leaves of its
 // walk separately, each in walk order, into a node and a leaf accumulator; its
@@ -962,8 +1072,9 @@ kb_force_group(BatchArgs a, uint32_t* __restrict__ work, const uint2* __restrict
 }
 
 template <bool EXACT, bool COUNT>
-__global__ void __launch_bounds__(kForceWarps * 32) kb_force(BatchArgs a, uint32_t* __restrict__ work) {
+__global__ void __launch_bounds__(kForceWarps * 32, 6) kb_force(BatchArgs a, uint32_t* __restrict__ work) {
     pdl_enter();
+    __shared__ RuleWindow win[kForceWarps];
     __shared__ uint32_t s_b;
     const uint32_t total = __ldg(&a.first[a.nsys]);
     for (;;) {
@@ -975,10 +1086,14 @@ __global__ void __launch_bounds__(kForceWarps * 32) kb_force(BatchArgs a, uint32
         const BatchBlock bb = batch_block(a, b);
         const SysDesc& d = *bb.d;
         const int f = d.passes & 1;
-        force_body<EXACT, COUNT>(bb.blk, d.idx[f], d.counters + kCtrValid, d.rec, d.skip, d.pos[bb.in],
-                                 d.vel[bb.in], d.pos[bb.out], d.vel[bb.out], d.acc, d.n_al, d.eps2, d.theta2, d.k,
-                                 d.hdt, d.cap, (unsigned long long*)(d.counters + kCtrStat),
-                                 d.ext ? d.ext + 4 * bb.out : nullptr);
+        auto walk = [&](auto ftz) {
+            force_body<EXACT, COUNT, decltype(ftz)::value, false>(
+                bb.blk, &win[threadIdx.x >> 5], nullptr, nullptr, d.idx[f], d.counters + kCtrValid, d.rec, d.skip,
+                d.pos[bb.in], d.vel[bb.in], d.pos[bb.out], d.vel[bb.out], d.acc, d.n_al, d.eps2, d.theta2, d.k, d.hdt,
+                d.cap, (unsigned long long*)(d.counters + kCtrStat), d.ext ? d.ext + 4 * bb.out : nullptr);
+        };
+        if (EXACT || rule_ftz(d.eps2)) walk(std::true_type{});
+        else walk(std::false_type{});
     }
 }
 
@@ -1064,8 +1179,20 @@ BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, bool quad, bool es
 template <bool EXACT>
 cudaError_t force_launch_impl(const ForceLaunch& f) {
     if (!f.group) {  // the reference's warp-vote walk
-        auto fn = f.count ? k_force<EXACT, true> : k_force<EXACT, false>;
+        const bool ftz = EXACT || rule_ftz(f.eps2);
         const int blocks = (int)((f.n_al / 32 + kForceWarps - 1) / kForceWarps);
+        if (f.n_al <= kRuleStagedMax) {
+            auto fn = f.count ? (ftz ? k_force_staged<EXACT, true, true> : k_force_staged<EXACT, true, false>)
+                              : (ftz ? k_force_staged<EXACT, false, true> : k_force_staged<EXACT, false, false>);
+            const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)sizeof(RuleTree));
+            if (e != cudaSuccess) return e;
+            return launch_shared(f.pdl, fn, blocks, kForceWarps * 32, (unsigned)sizeof(RuleTree), f.st, f.sidx,
+                                 f.counts, f.rec, f.skip, f.pos_in, f.vel_in, f.pos_out, f.vel_out, f.acc, f.n_al,
+                                 f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
+        }
+        auto fn = f.count ? (ftz ? k_force<EXACT, true, true> : k_force<EXACT, true, false>)
+                          : (ftz ? k_force<EXACT, false, true> : k_force<EXACT, false, false>);
         return launch(f.pdl, fn, blocks, kForceWarps * 32, f.st, f.sidx, f.counts, f.rec, f.skip, f.pos_in, f.vel_in,
                       f.pos_out, f.vel_out, f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
     }
