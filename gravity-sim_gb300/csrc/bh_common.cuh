@@ -31,14 +31,19 @@ struct Blk {
 };
 __device__ __forceinline__ Blk grid_blk() { return Blk{blockIdx.x, gridDim.x}; }
 
-// Programmatic dependent launch: every step kernel lets the next launch in its stream
-// start as soon as all of its blocks have begun, then waits until the kernel before it
-// has finished and its writes are visible.  Each kernel therefore still runs strictly
-// after its predecessor (and transitively after all earlier ones); only the launch
-// latency between them is hidden.  Without the launch attribute both are no-ops.
+// Programmatic dependent launch: every step kernel waits until the kernel before it has
+// finished and its writes are visible, and then lets the next launch in its stream start.
+// Each kernel therefore still runs strictly after its predecessor (and transitively after
+// all earlier ones); only the launch latency between them is hidden.  In this order the
+// next kernel's blocks start only once the kernel before this one has finished.  With the
+// trigger first they could start while kernels two and three back were still loading lines
+// into an L1 that their start had already cleared, and read those lines after they had been
+// rewritten: the node moments once saw a tree without internal nodes, from the line of
+// counters that the node scan had read before it wrote their number.  Without the launch
+// attribute both are no-ops.
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {

@@ -31,15 +31,6 @@ constexpr int kDirectBlock = 128;
 constexpr int kDirectTileJ = 64;
 constexpr int kDirectIpt = 2;  // default targets per thread (gs_shape.direct_targets: 2 or 4), in packed f32x2 pairs
 
-// Steps launched programmatically behind one another (direct_step): wait for the step
-// before, then let the next one start.  In this order the next step's blocks start only once
-// the step before this one has finished: the step after next writes what that one read, and
-// its lines could otherwise still enter an L1 that the next step's start has already cleared.
-__device__ __forceinline__ void chain_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // 1/sqrt of a softened squared distance.  d2 >= eps2, so with a normal eps2 (FTZ) it is
 // never subnormal and the flush-to-zero form gives the same bits; the plain form also
 // scales subnormal inputs, six more instructions per pair of targets.
@@ -323,7 +314,7 @@ __global__ void __launch_bounds__(kDirectSmallWarps * 32)
 k_direct_small(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
                float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
                uint32_t n_al, float eps2, float k, float hdt) {
-    chain_enter();
+    pdl_enter();
     __shared__ __align__(16) DirectSmallSmem<kDirectSmallWarps> g;
     direct_small_body<kDirectSmallWarps, KAHAN, FTZ>(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2,
                                                      k, hdt);
@@ -573,7 +564,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32)
 k_direct_rows(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
               float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec, uint32_t n_al,
               float eps2, float k, float hdt) {
-    chain_enter();
+    pdl_enter();
     __shared__ __align__(16) DirectRowsSmem<kRowsWarps> g;
     direct_rows_body<kRowsWarps>(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
 }
@@ -584,7 +575,7 @@ k_direct_fast(const float2* __restrict__ pos, const float2* __restrict__ vel, co
               float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
               uint32_t n_al, int chunks, uint32_t jchunk, float eps2, float k, float hdt, float4* __restrict__ partials,
               uint32_t* __restrict__ tickets) {
-    chain_enter();
+    pdl_enter();
     direct_fast_body<IPT, KAHAN, FTZ>(blockIdx.x, blockIdx.y, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, chunks,
                                       jchunk, eps2, k, hdt, partials, tickets);
 }
@@ -593,7 +584,7 @@ __global__ void __launch_bounds__(kRefThreads, 2)
 k_direct_ref(const float2* __restrict__ pos, const float2* __restrict__ vel, const float* __restrict__ mass,
              float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
              uint32_t n_al, float eps2, float k, float hdt) {
-    chain_enter();
+    pdl_enter();
     __shared__ __align__(16) DirectRefSmem g;
     direct_ref_body(g, blockIdx.x, pos, vel, mass, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt);
 }
