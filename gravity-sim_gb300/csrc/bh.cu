@@ -521,13 +521,22 @@ SortPassFn sort_pass_kernel_kpt(bool identity, uint32_t lb) {
         default: return identity ? k_sort_pass<true, KPT, 32> : k_sort_pass<false, KPT, 32>;
     }
 }
-SortPassFn sort_pass_kernel(bool identity, const gs_shape& sh) {
-    return sh.sort_keys_per_thread == 8 ? sort_pass_kernel_kpt<8>(identity, sh.sort_lookback)
-                                        : sort_pass_kernel_kpt<16>(identity, sh.sort_lookback);
+// Keys per thread of a system sorted alone.  A tile's ranks are a serial chain over a thread's
+// keys, and up to kSortSmallMax keys the look-back over the tiles is one round trip however
+// small they are, so a small system takes tiles of 1024 keys whatever its shape says (three
+// passes over 10,000 keys: 22 us, in tiles of 4096 32; over 100,000: 26 and 36).
+constexpr uint64_t kSortSmallMax = 131072;
+inline uint32_t sort_kpt(uint64_t n, const gs_shape& sh) {
+    return n <= kSortSmallMax ? 4u : sh.sort_keys_per_thread == 8 ? 8u : 16u;
 }
-// radix-sort tiles of n keys under a shape
-inline uint32_t sort_tiles_of(uint64_t n, const gs_shape& sh) {
-    const uint64_t tile = (uint64_t)kSortThreads * (sh.sort_keys_per_thread == 8 ? 8 : 16);
+SortPassFn sort_pass_kernel(bool identity, uint32_t kpt, const gs_shape& sh) {
+    return kpt == 4   ? sort_pass_kernel_kpt<4>(identity, sh.sort_lookback)
+           : kpt == 8 ? sort_pass_kernel_kpt<8>(identity, sh.sort_lookback)
+                      : sort_pass_kernel_kpt<16>(identity, sh.sort_lookback);
+}
+// radix-sort tiles of n keys, kpt per thread
+inline uint32_t sort_tiles_of(uint64_t n, uint32_t kpt) {
+    const uint64_t tile = (uint64_t)kSortThreads * kpt;
     return (uint32_t)((n + tile - 1) / tile);
 }
 
@@ -1182,7 +1191,7 @@ void bh_carve(gs_sim* s) {
     // 30-bit keys), 20-bit keys + removal bit in the fixed box (3 passes)
     w.passes = bbox ? (2 * w.depth + 7) / 8 : 3;
     w.cap = bh_capacity(w.depth, n);
-    w.sort_tiles = (uint32_t)((n + kSortThreads * 8 - 1) / (kSortThreads * 8));  // status for the smallest tiles
+    w.sort_tiles = sort_tiles_of(n, n <= kSortSmallMax ? 4 : 8);  // status for the smallest tiles
     w.scan_tiles = (uint32_t)((n + 1 + kScanTile - 1) / kScanTile);
     for (int b = 0; b < 2; ++b) {
         sim_carve(s, (void**)&w.keys[b], n * sizeof(uint32_t));
@@ -1296,10 +1305,11 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     count_launch(s);
     stage_end(s, kStageKeys, profile);
     stage_begin(s, kStageSort, profile);
+    const uint32_t kpt = sort_kpt(n, s->shape);
     for (int ps = 0; ps < w.passes; ++ps) {
         const int a = ps & 1, b = a ^ 1;
         uint32_t* status = w.sort_status + (size_t)ps * w.sort_tiles * 256;
-        GS_TRY_LAUNCH(launch(next_pdl(), sort_pass_kernel(ps == 0, s->shape), (int)sort_tiles_of(n, s->shape),
+        GS_TRY_LAUNCH(launch(next_pdl(), sort_pass_kernel(ps == 0, kpt, s->shape), (int)sort_tiles_of(n, kpt),
                              kSortThreads, st, (const uint32_t*)w.keys[a], (const uint32_t*)(ps == 0 ? nullptr : w.idx[a]),
                              w.keys[b], w.idx[b], n, 8 * ps, (const uint32_t*)(w.hist + 256 * ps), status,
                              ctr + kCtrSort + ps, s->d_err));
@@ -1728,7 +1738,7 @@ void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_s
     }
     blocks[kTabGrid] = (uint32_t)grid_for(n, 256);
     blocks[kTabKeys] = (uint32_t)keygen_blocks(n);
-    blocks[kTabSort] = sort_tiles_of(n, shape);
+    blocks[kTabSort] = sort_tiles_of(n, shape.sort_keys_per_thread == 8 ? 8 : 16);
     blocks[kTabScan] = w.scan_tiles;
     blocks[kTabMom] = w.mom_blocks;
     blocks[kTabOne] = 1;
