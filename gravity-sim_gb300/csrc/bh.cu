@@ -1688,8 +1688,7 @@ __global__ void __launch_bounds__(512) kb_top_sums(BatchArgs a) {
 
 // Descriptor and per-stage block counts of one Barnes-Hut system; the counts are the
 // plain path's, except that the bounding box uses no more blocks than its particles fill.
-void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& shape,
-                   uint32_t force_warps) {
+void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& shape) {
     const BHWork& w = s->bh;
     d.keys[0] = w.keys[0];
     d.keys[1] = w.keys[1];
@@ -1742,9 +1741,9 @@ void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_s
     blocks[kTabScan] = w.scan_tiles;
     blocks[kTabMom] = w.mom_blocks;
     blocks[kTabOne] = 1;
-    const uint64_t per_block = (s->p.flags & GS_FLAG_GROUP_WALK) ? (uint64_t)force_warps * kGroupSize
-                                                                   : (uint64_t)kForceWarps * 32;
-    blocks[kTabForce] = (uint32_t)((n + per_block - 1) / per_block);
+    // the group walk's warps take single groups, the warp-vote walk's blocks a block's particles
+    const uint64_t per_unit = (s->p.flags & GS_FLAG_GROUP_WALK) ? (uint64_t)kGroupSize : (uint64_t)kForceWarps * 32;
+    blocks[kTabForce] = (uint32_t)((n + per_unit - 1) / per_unit);
 }
 
 namespace {
@@ -1782,6 +1781,7 @@ static BatchForceLaunch batch_force(const BatchPlan& p, uint32_t step, cudaStrea
 
 int bh_batch_force_grid(const BatchPlan& p) {
     BatchForceLaunch b = batch_force(p, 0, nullptr);
+    b.units = p.total[kTabForce];
     int grid = 0;
     const cudaError_t e = (p.exact ? batch_force_launch_exact : batch_force_launch_fast)(b, &grid);
     return e == cudaSuccess && grid > 0 ? grid : 152;
@@ -1827,9 +1827,9 @@ cudaError_t bh_batch_step(const BatchPlan& p, uint32_t step, cudaStream_t st, bo
             GS_TRY_LAUNCH(launch(true, kb_level_sums, (int)p.total[kTabGrid], 256, st, args(kTabGrid), lv));
         GS_TRY_LAUNCH(launch(true, kb_top_sums, (int)p.total[kTabOne], 512, st, args(kTabOne)));
     }
-    const int fg = p.force_grid < (int)p.total[kTabForce] ? p.force_grid : (int)p.total[kTabForce];
     BatchForceLaunch b = batch_force(p, step, st);
-    b.grid = fg;
+    b.grid = p.force_grid < (int)p.total[kTabForce] ? p.force_grid : (int)p.total[kTabForce];
+    b.units = p.total[kTabForce];
     auto run = p.exact ? batch_force_launch_exact : batch_force_launch_fast;
     if (estimate && p.group && p.quad) {  // |a| of the groups that have none (members that just joined or were reset)
         BatchForceLaunch e = b;

@@ -219,37 +219,121 @@ k_force_staged(const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ c
 
 // ------------------------------------------------------------------------------------
 // accurate-mode traversal (no counterpart in the reference): the 64 particles of 64
-// consecutive sorted slots share one walk, run by one warp (two particles per lane); 32
-// records are tested at once (one per lane) against the bounding boxes of the group;
-// accepted nodes and runs of particle leaves are collected and every lane then sums them
-// for its two particles with packed f32x2 instructions (quadrupole term for nodes).
+// consecutive sorted slots share one walk: 32 records are tested at once (one per lane)
+// against the bounding boxes of the group; accepted nodes and runs of particle leaves are
+// collected, and every lane sums them for its two particles with packed f32x2 instructions
+// (quadrupole term for nodes).
+//
+// One warp does both (SPLIT false), or two share a group: a walking warp that tests and
+// collects, and a summing warp, the lists going from one to the other through two slots in
+// shared memory.  One warp spends half its time in each: at N = 20,000, where a scheduler
+// has at most one warp, 46 of 103 thousand cycles a group in the walk's chain of L2 round trips
+// and 53 in the sums' dependent instructions; on two warps the halves overlap.
 // ------------------------------------------------------------------------------------
 // Records still to test.  Pops take the top 32 and push at most four internal children
 // each, one level deeper, so the stack holds at most one block of <= 128 entries per level
-// and blocks of strictly increasing level: <= 96 * D + 128 = 1568 for D = 15.  Overflow
-// is still checked and reported.
+// and blocks of strictly increasing level: <= 96 * D + 128 = 1568 for D = 15 (checked and
+// reported).  The walks of a 500k-particle spiral stay below 230, so shared memory holds the
+// top 256 entries and a deeper stack's bottom goes to the walking warp's local memory, 128
+// entries at a time.
 constexpr int kStackCap = 1568;
 static_assert(kStackCap >= 96 * (kBBoxMaxBits > kFixedDepth ? kBBoxMaxBits : kFixedDepth) + 128, "walk stack bound");
-// Accepted nodes and runs of particle leaves collected between evaluations: 160 / 128
-// (long lists) or 96 / 64 (short lists, gs_shape.force_short_lists); a pop adds at most
-// 32 nodes and 64 runs.
+constexpr int kStackWindow = 256, kStackSpill = 128;          // of a walk
+constexpr int kPairStackWindow = 512, kPairStackSpill = 256;  // of a costly group's (64-record pops)
+constexpr int kSinglePerSm = 20, kSplitPerSm = 8;  // resident groups the registers are cut for
+
+// The bottom of a stack that outgrew its window: lane l keeps entries l, 32 + l, ...
+template <int CAP, int SPILL>
+struct StackSpill {
+    uint32_t e[(CAP + SPILL - 1) / SPILL * SPILL / 32];
+    uint32_t count = 0;  // entries below the window
+
+    // Moves the window's lowest SPILL entries out (size > SPILL of them).
+    __device__ __forceinline__ uint32_t save(uint32_t* stack, uint32_t size, int lane) {
+        for (uint32_t j = 0; j < SPILL; j += 32) e[(count + j) / 32] = stack[j + lane];
+        for (uint32_t j = SPILL; j < size; j += 32) {  // upwards: a row's target lies below it
+            const uint32_t v = j + lane < size ? stack[j + lane] : 0u;
+            __syncwarp();
+            if (j + lane < size) stack[j + lane - SPILL] = v;
+            __syncwarp();
+        }
+        count += SPILL;
+        return size - SPILL;
+    }
+    // Moves them back below the size entries of the window (size <= 64).
+    __device__ __forceinline__ uint32_t restore(uint32_t* stack, uint32_t size, int lane) {
+        const uint32_t v0 = (uint32_t)lane < size ? stack[lane] : 0u, v1 = lane + 32u < size ? stack[lane + 32] : 0u;
+        __syncwarp();
+        count -= SPILL;
+        if ((uint32_t)lane < size) stack[SPILL + lane] = v0;
+        if (lane + 32u < size) stack[SPILL + 32 + lane] = v1;
+        for (uint32_t j = 0; j < SPILL; j += 32) stack[j + lane] = e[(count + j) / 32];
+        __syncwarp();
+        return size + SPILL;
+    }
+};
 
 // Evaluation order.  Each particle sums the accepted nodes and the particle leaves of its
 // walk separately, each in walk order, into a node and a leaf accumulator; its
-// acceleration is node + leaf.  How the warp batches its evaluations therefore does not
-// change a bit of the result.
-template <int NODE, int ITEM>
+// acceleration is node + leaf.  How the lists are cut into slots therefore does not change
+// a bit of the result.
+//
+// A walk's lists are summed (SPLIT: passed on) once they hold NODE nodes or ITEM leaf runs (a
+// pop adds at most 32 nodes and 64 runs).
+template <int NODE, int ITEM, int SLOTS>
 struct GroupSmem {
-    static constexpr int kNode = NODE, kItem = ITEM;
-    static_assert(NODE >= 64 && ITEM >= 64 && ITEM % 32 == 0, "a pop adds <= 32 nodes and <= 64 leaf runs");
-    uint32_t stack[kStackCap];
-    uint32_t node[NODE];          // accepted node records
-    uint32_t it_start[ITEM];      // runs of particle leaves: first record
-    uint32_t it_count[ITEM];      // record count
-    uint32_t off[ITEM];           // exclusive record offsets of the runs
-    float cx[32], cy[32], cm[32];     // one chunk of gathered records: centre of mass (or particle), mass
-    float qxx[32], qxy[32], qyy[32], mt[32];  // node terms 7.5 S and -1.5 tr(S) of node records
+    static constexpr int kFullNode = NODE, kFullItem = ITEM, kNode = NODE + 32, kItem = (ITEM + 64 + 31) / 32 * 32;
+    static constexpr bool kSplit = SLOTS == 2;
+    static_assert(kItem % 32 == 0, "whole rows of runs");
+    uint32_t stack[kStackWindow];
+    struct Slot {
+        uint32_t node[kNode];   // accepted node records
+        uint2 run[kItem];       // runs of particle leaves: first record, count
+        uint32_t nodes, runs, last;
+    } slot[SLOTS];
+    uint64_t full[2], empty[2];  // SPLIT: mbarriers of the slots
+    uint32_t off[kItem];        // exclusive record offsets of a slot's runs
+    // One chunk of gathered records: {x, y, m, -1.5 tr(S)}, 7.5 {Sxx, Sxy, Syy}.  A scalar
+    // of a record costs one register move to pair it for the two particles; stored as
+    // pairs it would cost a broadcast load's bandwidth, which goes by the bytes delivered.
+    float4 ca[32], cb[32];
 };
+
+// The two warps of a walk hand slots over through mbarriers in shared memory (full and empty
+// again, one arrival each).  Named barriers would do the same, but an SM has 64 of them,
+// and sixteen walks with four each (or a block that reserves all sixteen ids because they
+// are computed) leave no room: 14 of 32 warps resident, 360 us at N = 500,000.
+__device__ __forceinline__ uint32_t bar_address(const uint64_t& bar) { return (uint32_t)__cvta_generic_to_shared(&bar); }
+__device__ __forceinline__ void bar_init(uint64_t& bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_address(bar)) : "memory");
+}
+// The warp's earlier reads and writes of the slot come before the other side's.
+__device__ __forceinline__ void bar_pass(uint64_t& bar, int lane) {
+    __syncwarp();
+    if (lane == 0)
+        asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.release.cta.shared::cta.b64 t, [%0];\n\t}" ::"r"(bar_address(bar))
+                     : "memory");
+}
+// Waits for the arrival that ends phase `parity`; false after kSpinLimit tries.
+__device__ __forceinline__ bool bar_wait(const uint64_t& bar, uint32_t parity) {
+    uint32_t done = 0;
+    for (uint32_t spin = 0; !done && spin < kSpinLimit; ++spin)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(bar_address(bar)), "r"(parity)
+                     : "memory");
+    return __all_sync(0xffffffffu, done != 0);
+}
+
+// Barrier of a walk's two warps (a named one, by a constant so that a block reserves no more
+// than its walks need).
+__device__ __forceinline__ void pair_sync(int walk) {
+    if (walk == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+    else if (walk == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+    else if (walk == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+    else asm volatile("bar.sync 4, 64;" ::: "memory");
+}
 
 // One record (x, y, m) on the lane's two particles (P = their x, Q = their y):
 // d = (x, y) - p, d2 = dx^2 + dy^2 + eps^2, a += d * (((m r) r) r) with r = 1/sqrt(d2),
@@ -291,101 +375,112 @@ __device__ __forceinline__ void quadrupole_x2(float x, float y, float m, float q
     acy = fma2(r3, iy, acy);
 }
 
+// A gathered node's record and moments as a chunk's entry.
+template <bool QUAD>
+__device__ __forceinline__ void stage_node(float4* ca, float4* cb, int lane, const float4& q, const float4& qq) {
+    ca[lane] = make_float4(q.x, q.y, q.z, QUAD ? -1.5f * (qq.x + qq.z) : 0.0f);
+    if (QUAD) cb[lane] = make_float4(7.5f * qq.x, 7.5f * qq.y, 7.5f * qq.z, 0.0f);
+}
+// Entries [klo, khi) of a chunk on the lane's two particles.
+template <bool EXACT, bool QUAD>
+__device__ __forceinline__ void sum_chunk(const float4* ca, const float4* cb, uint32_t klo, uint32_t khi, float2 P,
+                                          float2 Q, float2 E2, float2& acx, float2& acy) {
+#pragma unroll 4
+    for (uint32_t j = klo; j < khi; ++j) {
+        const float4 a = ca[j];
+        if (QUAD) {
+            const float4 b = cb[j];
+            quadrupole_x2<EXACT>(a.x, a.y, a.z, b.x, b.y, b.z, a.w, P, Q, E2, acx, acy);
+        } else {
+            monopole_x2<EXACT>(a.x, a.y, a.z, P, Q, E2, acx, acy);
+        }
+    }
+}
+
 // Sum the count accepted nodes (quadrupole term with QUAD) for the lane's two particles,
 // 32 at a time: lane l loads node l of the next chunk while the current one is summed.
-template <bool EXACT, bool QUAD, class SM>
-__device__ __forceinline__ void eval_nodes(SM& g, uint32_t count, const float4* __restrict__ rec,
-                                           const float4* __restrict__ quad, float2 P, float2 Q, float2 E2,
-                                           float2& acx, float2& acy, int lane) {
+template <bool EXACT, bool QUAD>
+__device__ __forceinline__ void eval_nodes(const uint32_t* node, float4* ca, float4* cb, uint32_t count,
+                                           const float4* __restrict__ rec, const float4* __restrict__ quad, float2 P,
+                                           float2 Q, float2 E2, float2& acx, float2& acy, int lane) {
     if (!count) return;
     float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f), qq = q;
     if ((uint32_t)lane < count) {
-        const uint32_t r = g.node[lane];
+        const uint32_t r = node[lane];
         q = __ldg(&rec[r]);
         if (QUAD) qq = __ldg(&quad[r]);
     }
     for (uint32_t f0 = 0; f0 < count; f0 += 32) {
-        const uint32_t m = min(count - f0, 32u);
-        g.cx[lane] = q.x;
-        g.cy[lane] = q.y;
-        g.cm[lane] = q.z;
-        if (QUAD) {
-            g.qxx[lane] = 7.5f * qq.x;
-            g.qxy[lane] = 7.5f * qq.y;
-            g.qyy[lane] = 7.5f * qq.z;
-            g.mt[lane] = -1.5f * (qq.x + qq.z);
-        }
+        __syncwarp();
+        stage_node<QUAD>(ca, cb, lane, q, qq);
         __syncwarp();
         const uint32_t fn = f0 + 32 + lane;
         if (fn < count) {
-            const uint32_t r = g.node[fn];
+            const uint32_t r = node[fn];
             q = __ldg(&rec[r]);
             if (QUAD) qq = __ldg(&quad[r]);
         }
-#pragma unroll 4
-        for (uint32_t j = 0; j < m; ++j) {
-            if (QUAD)
-                quadrupole_x2<EXACT>(g.cx[j], g.cy[j], g.cm[j], g.qxx[j], g.qxy[j], g.qyy[j], g.mt[j], P, Q, E2, acx,
-                                     acy);
-            else
-                monopole_x2<EXACT>(g.cx[j], g.cy[j], g.cm[j], P, Q, E2, acx, acy);
-        }
-        __syncwarp();
+        sum_chunk<EXACT, QUAD>(ca, cb, 0, min(count - f0, 32u), P, Q, E2, acx, acy);
     }
 }
 
-// Record f of the leaf runs (last run with off <= f).
-template <class SM>
-__device__ __forceinline__ float4 gather_leaf(const SM& g, uint32_t n_items, uint32_t f,
-                                              const float4* __restrict__ rec) {
-    uint32_t lo = 0, hi = n_items - 1;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (g.off[mid] <= f) lo = mid;
-        else hi = mid - 1;
-    }
-    return __ldg(&rec[g.it_start[lo] + (f - g.off[lo])]);
-}
-
-// Sum the particle leaves of the n_items runs as monopoles, 32 records at a time.
-template <bool EXACT, class SM>
-__device__ __forceinline__ void eval_leaves(SM& g, uint32_t n_items, const float4* __restrict__ rec,
-                                            float2 P, float2 Q, float2 E2, float2& acx, float2& acy, int lane) {
-    if (!n_items) return;
-    // exclusive record offsets of all runs: lane l owns runs [4l, 4l + 4)
-    uint32_t c4[SM::kItem / 32], sum = 0;
+// Exclusive record offsets of n_items leaf runs, and their total: lane l owns runs
+// [K l, K l + K).
+template <int K>
+__device__ __forceinline__ uint32_t run_offsets(const uint2* run, uint32_t* off, uint32_t n_items, int lane) {
+    uint32_t cnt[K], sum = 0;
 #pragma unroll
-    for (int t = 0; t < SM::kItem / 32; ++t) {
-        const uint32_t it = lane * (SM::kItem / 32) + t;
-        c4[t] = it < n_items ? g.it_count[it] : 0u;
-        sum += c4[t];
+    for (int t = 0; t < K; ++t) {
+        const uint32_t it = (uint32_t)lane * K + t;
+        cnt[t] = it < n_items ? run[it].y : 0u;
+        sum += cnt[t];
     }
     uint32_t x = sum;
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
-    uint32_t run = x - sum;
+    uint32_t at = x - sum;
 #pragma unroll
-    for (int t = 0; t < SM::kItem / 32; ++t) {
-        g.off[lane * (SM::kItem / 32) + t] = run;
-        run += c4[t];
+    for (int t = 0; t < K; ++t) {
+        off[lane * K + t] = at;
+        at += cnt[t];
     }
-    __syncwarp();
+    return __shfl_sync(0xffffffffu, x, 31);
+}
+
+// Record f0 + lane of the flattened leaf runs (if below total); r0 is the run that holds
+// record f0, and is moved on to the one that holds f0 + 32.  The runs that start inside
+// the chunk mark a bit each, and a lane's run is r0 plus the marks up to it.
+__device__ __forceinline__ float4 gather_leaf(const uint2* run, const uint32_t* off, uint32_t n_items, uint32_t f0,
+                                              uint32_t total, uint32_t& r0, const float4* __restrict__ rec, int lane) {
+    const uint32_t r = r0 + 1 + lane, o = r < n_items ? off[r] : 0xffffffffu;
+    const uint32_t marks = __reduce_or_sync(0xffffffffu, o - f0 < 32u ? 1u << (o - f0) : 0u);
+    const uint32_t mine = r0 + __popc(marks & (0xffffffffu >> (31 - lane)));
     float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if ((uint32_t)lane < total) q = gather_leaf(g, n_items, lane, rec);
+    if (f0 + lane < total) q = __ldg(&rec[run[mine].x + (f0 + lane - off[mine])]);
+    r0 += __popc(marks);
+    if (r0 + 1 < n_items && off[r0 + 1] == f0 + 32) ++r0;
+    return q;
+}
+
+// Sum the particle leaves of the n_items runs as monopoles, 32 records at a time.
+template <bool EXACT, int ITEM>
+__device__ __forceinline__ void eval_leaves(const uint2* run, uint32_t* off, float4* ca, uint32_t n_items,
+                                            const float4* __restrict__ rec, float2 P, float2 Q, float2 E2, float2& acx,
+                                            float2& acy, int lane) {
+    if (!n_items) return;
+    __syncwarp();  // the previous slot's offsets have been read
+    const uint32_t total = run_offsets<ITEM / 32>(run, off, n_items, lane);
+    __syncwarp();
+    uint32_t r0 = 0;
+    float4 q = gather_leaf(run, off, n_items, 0, total, r0, rec, lane);
     for (uint32_t f0 = 0; f0 < total; f0 += 32) {
-        const uint32_t m = min(total - f0, 32u);
-        g.cx[lane] = q.x;
-        g.cy[lane] = q.y;
-        g.cm[lane] = q.z;
         __syncwarp();
-        const uint32_t fn = f0 + 32 + lane;
-        if (fn < total) q = gather_leaf(g, n_items, fn, rec);
-#pragma unroll 4
-        for (uint32_t j = 0; j < m; ++j) monopole_x2<EXACT>(g.cx[j], g.cy[j], g.cm[j], P, Q, E2, acx, acy);
+        ca[lane] = q;
         __syncwarp();
+        if (f0 + 32 < total) q = gather_leaf(run, off, n_items, f0 + 32, total, r0, rec, lane);
+        sum_chunk<EXACT, false>(ca, nullptr, 0, min(total - f0, 32u), P, Q, E2, acx, acy);
     }
 }
 
@@ -520,76 +615,72 @@ __device__ __forceinline__ void group_boxes(const uint32_t* __restrict__ skey, u
     }
 }
 
-// ESTIMATE: the |a| estimate pass of the relative criterion.  A group whose particles all
-// have a previous |a| returns at once; any other group walks with the theta test and
-// writes only the |a| of its particles (no integration), which the following normal pass
-// then opens nodes by.
-template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, int WARPS, class SM>
-__device__ __forceinline__ void force_group_body(
-    Blk blk, SM& g, const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ skey,
-    const uint32_t* __restrict__ counts, const float4* __restrict__ rec, const uint32_t* __restrict__ skip,
-    const float4* __restrict__ quad, const uint4* __restrict__ kids, const float2* __restrict__ pos_in,
-    const float2* __restrict__ vel_in, float2* __restrict__ pos_out, float2* __restrict__ vel_out,
-    float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float theta2, float k, float hdt, uint32_t cap,
-    unsigned long long* __restrict__ stat, int* __restrict__ err, float* __restrict__ amag, float alpha,
-    float floor2, uint32_t* __restrict__ ext, const uint8_t* __restrict__ heavy) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t group = blk.id * WARPS + warp;
-    const uint32_t nv = counts[0];
-    const uint32_t T = min(nv + counts[1], cap);
-    const uint32_t g0 = group * kGroupSize;
-    if (g0 >= nv || T == 0) return;
-    if (ESTIMATE && !amag) return;  // a batch member without the relative criterion
-    if (heavy && heavy[group]) return;  // a costly group: walked by a warp pair (force_pair_body)
-    // particles: slot g0 + lane (.x of every pair) and g0 + 32 + lane (.y)
-    const uint32_t s0 = g0 + lane, s1 = s0 + 32;
-    const uint32_t i0 = s0 < nv ? sidx[s0] : 0u, i1 = s1 < nv ? sidx[s1] : 0u;
-    const bool v0 = s0 < nv && i0 < n_al, v1 = s1 < nv && i1 < n_al;  // i < n_al unless the sort failed
-    const float2 p0 = v0 ? pos_in[i0] : make_float2(0.0f, 0.0f);
-    const float2 p1 = v1 ? pos_in[i1] : make_float2(0.0f, 0.0f);
+// What a group's two warps read of its system.
+struct GroupSys {
+    const uint32_t *sidx, *skey, *counts;
+    const float4* rec;
+    const uint32_t* skip;
+    const float4* quad;
+    const uint4* kids;
+    const float2 *pos_in, *vel_in;
+    float2 *pos_out, *vel_out, *acc_rec;
+    uint32_t n_al;
+    float eps2, theta2, k, hdt;
+    uint32_t cap;
+    unsigned long long* stat;
+    int* err;
+    float* amag;
+    float alpha, floor2;
+    uint32_t* ext;
+    const uint8_t* heavy;
+};
+
+// The walk of a group: tests the records; flush(slot, nodes, runs, done) takes the lists,
+// slot by slot, and leaves the next slot free (false: a wait ran out).
+template <bool COUNT, bool ESTIMATE, class SM, class Flush>
+__device__ __forceinline__ bool group_walk(const GroupSys& y, SM& g, uint32_t nv, uint32_t g0, uint32_t s0,
+                                           uint32_t s1, bool v0, bool v1, float2 p0, float2 p1, bool unknown, float a0,
+                                           float a1, int lane, Flush&& flush) {
+    const float4* __restrict__ rec = y.rec;
+    const uint4* __restrict__ kids = y.kids;
     float bx0[4], bx1[4], by0[4], by1[4];
-    group_boxes(skey, g0, nv, s0, s1, v0, v1, p0, p1, bx0, bx1, by0, by1);
-    // Relative criterion: the smallest previous |a| of the group, NaN when any is unknown
-    // (then the group takes the theta test).  Each group reads and rewrites only its own
-    // particles' |a|, so one buffer serves as input and output.
+    group_boxes(y.skey, g0, nv, s0, s1, v0, v1, p0, p1, bx0, bx1, by0, by1);
+    // Relative criterion: the smallest previous |a| of the group (when any is unknown the
+    // group takes the theta test).  Each group reads and rewrites only its own particles'
+    // |a|, so one buffer serves as input and output.
     bool relative = false;
     float tol2 = 0.0f;
-    if (amag) {
-        const float a0 = v0 ? amag[i0] : INFINITY, a1 = v1 ? amag[i1] : INFINITY;
-        const bool unknown = __any_sync(0xffffffffu, isnan(a0) || isnan(a1));
-        if (ESTIMATE && !unknown) return;  // warp-uniform: nothing to estimate
+    if (y.amag) {
         float amin = fminf(a0, a1);
         for (int o = 16; o; o >>= 1) amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
         relative = !ESTIMATE && !unknown;
-        const float tol = alpha * amin;
+        const float tol = y.alpha * amin;
         tol2 = tol * tol;
     }
-    const float2 P = make_float2(p0.x, p1.x), Q = make_float2(p0.y, p1.y), E2 = make_float2(eps2, eps2);
-    // node and leaf accumulators of the two particles (.x particle 0, .y particle 1)
-    float2 anx = make_float2(0.0f, 0.0f), any = anx, alx = anx, aly = anx;
+    const float eps2 = y.eps2, floor2 = y.floor2, theta2 = y.theta2;
     unsigned long long n_int = 0, n_test = 0, n_node = 0;
-    uint32_t size = 0, n_nodes = 0, n_items = 0;
-    if (skip[0] == 1u) {  // a single particle: the root is its leaf
-        if (lane == 0) {
-            g.it_start[0] = 0u;
-            g.it_count[0] = 1u;
-        }
+    StackSpill<kStackCap, kStackSpill> spill;
+    uint32_t size = 0, n_nodes = 0, n_items = 0, passed = 0;  // slots passed on
+    const bool single = y.skip[0] == 1u;  // a single particle: the root is its leaf
+    if (single) {
+        if (lane == 0) g.slot[0].run[0] = make_uint2(0u, 1u);
         n_items = 1;
     } else {
         if (lane == 0) g.stack[0] = 0u;
         size = 1;
     }
     __syncwarp();
-
-    while (size > 0) {
-        if (n_nodes > (uint32_t)(SM::kNode - 32)) {
-            eval_nodes<EXACT, QUAD, SM>(g, n_nodes, rec, quad, P, Q, E2, anx, any, lane);
-            n_nodes = 0;
+    const uint32_t lt = (1u << lane) - 1u;
+    for (;;) {
+        const bool done = size == 0 && spill.count == 0;
+        if (done || n_nodes > (uint32_t)SM::kFullNode || n_items > (uint32_t)SM::kFullItem) {
+            if (!flush(passed & 1u, n_nodes, n_items, done)) return false;
+            ++passed;
+            n_nodes = n_items = 0;
+            if (done) break;
         }
-        if (n_items > (uint32_t)(SM::kItem - 64)) {
-            eval_leaves<EXACT, SM>(g, n_items, rec, P, Q, E2, alx, aly, lane);
-            n_items = 0;
-        }
+        if (size < 32u && spill.count) size = spill.restore(g.stack, size, lane);
+        typename SM::Slot& sl = g.slot[SM::kSplit ? passed & 1u : 0u];
         const uint32_t np = min(size, 32u);
         const uint32_t base = size - np;
         const bool act = lane < (int)np;
@@ -599,67 +690,144 @@ __device__ __forceinline__ void force_group_body(
         if (COUNT) n_test += np;
         RecTest r{};
         if (act) test_record(n, rec, kids, bx0, bx1, by0, by1, eps2, relative, tol2, floor2, theta2, r);
-        const uint32_t a0 = r.a0, c0 = r.c0, a1 = r.a1, c1 = r.c1, nl = r.nl, nn = r.nn;
-        const uint32_t pu0 = r.pu[0], pu1 = r.pu[1], pu2 = r.pu[2], pu3 = r.pu[3];
-        uint32_t npu = r.npu;
-        // offsets in lane order, three counts in one scan: nodes <= 32, runs <= 64 and
-        // pushes <= 128 in warp total, so the 8/8/16-bit fields never carry
-        const uint32_t mine = nn | (nl << 8) | (npu << 16);
-        uint32_t x = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+        // offsets in lane order from the ballots of the counts' bits: nodes 0..1, runs 0..2,
+        // pushes 0..4
+        const uint32_t bn = __ballot_sync(0xffffffffu, r.nn);
+        const uint32_t bl0 = __ballot_sync(0xffffffffu, r.nl & 1u), bl1 = __ballot_sync(0xffffffffu, r.nl & 2u);
+        const uint32_t bp0 = __ballot_sync(0xffffffffu, r.npu & 1u), bp1 = __ballot_sync(0xffffffffu, r.npu & 2u);
+        const uint32_t bp2 = __ballot_sync(0xffffffffu, r.npu & 4u);
+        const uint32_t ptot = __popc(bp0) + 2 * __popc(bp1) + 4 * __popc(bp2);
+        if (size + ptot > (uint32_t)kStackWindow) size = spill.save(g.stack, size, lane);
+        uint32_t npu = r.npu, pushed = ptot;
+        if (spill.count + size + ptot > (uint32_t)kStackCap) {  // beyond the depth bound: report, do not overrun
+            if (lane == 0) atomicOr(y.err, kErrTree);
+            pushed = npu = 0;
         }
-        const uint32_t ex = x - mine, tot = __shfl_sync(0xffffffffu, x, 31);
-        const uint32_t noff = ex & 0xffu, loff = (ex >> 8) & 0xffu, poff = ex >> 16;
-        const uint32_t ntot = tot & 0xffu, ltot = (tot >> 8) & 0xffu;
-        uint32_t ptot = tot >> 16;
-        if (size + ptot > (uint32_t)kStackCap) {  // beyond the depth bound: report, do not overrun
-            if (lane == 0) atomicOr(err, kErrTree);
-            ptot = 0;
-            npu = 0;
-        }
-        if (nn) g.node[n_nodes + noff] = n;
-        if (nl > 0) {
-            g.it_start[n_items + loff] = a0;
-            g.it_count[n_items + loff] = c0;
-        }
-        if (nl > 1) {
-            g.it_start[n_items + loff + 1] = a1;
-            g.it_count[n_items + loff + 1] = c1;
+        if (r.nn) sl.node[n_nodes + __popc(bn & lt)] = n;
+        if (r.nl) {
+            uint2* run = sl.run + n_items + __popc(bl0 & lt) + 2 * __popc(bl1 & lt);
+            run[0] = make_uint2(r.a0, r.c0);
+            if (r.nl > 1) run[1] = make_uint2(r.a1, r.c1);
         }
         if (COUNT) {
-            n_int += nn + (nl > 0 ? c0 : 0u) + (nl > 1 ? c1 : 0u);
-            n_node += nn;
+            n_int += r.nn + (r.nl > 0 ? r.c0 : 0u) + (r.nl > 1 ? r.c1 : 0u);
+            n_node += r.nn;
         }
-        uint32_t* dst = g.stack + size + poff;
-        if (npu > 0) dst[0] = pu0;
-        if (npu > 1) dst[1] = pu1;
-        if (npu > 2) dst[2] = pu2;
-        if (npu > 3) dst[3] = pu3;
-
-        n_nodes += ntot;
-        n_items += ltot;
-        size += ptot;
+        uint32_t* dst = g.stack + size + __popc(bp0 & lt) + 2 * __popc(bp1 & lt) + 4 * __popc(bp2 & lt);
+        if (npu > 0) dst[0] = r.pu[0];
+        if (npu > 1) dst[1] = r.pu[1];
+        if (npu > 2) dst[2] = r.pu[2];
+        if (npu > 3) dst[3] = r.pu[3];
+        n_nodes += __popc(bn);
+        n_items += __popc(bl0) + 2 * __popc(bl1);
+        size += pushed;
         __syncwarp();
     }
-    eval_nodes<EXACT, QUAD, SM>(g, n_nodes, rec, quad, P, Q, E2, anx, any, lane);
-    eval_leaves<EXACT, SM>(g, n_items, rec, P, Q, E2, alx, aly, lane);
     if (COUNT) {
-        if (skip[0] == 1u && lane == 0) n_int += 1;
+        if (single && lane == 0) n_int += 1;
         for (int o = 16; o; o >>= 1) {
             n_int += __shfl_xor_sync(0xffffffffu, n_int, o);
             n_node += __shfl_xor_sync(0xffffffffu, n_node, o);
         }
         const unsigned long long nval = __popc(__ballot_sync(0xffffffffu, v0)) + __popc(__ballot_sync(0xffffffffu, v1));
         if (lane == 0) {
-            atomicAdd(&stat[0], n_int * nval);
-            atomicAdd(&stat[1], n_test);
-            atomicAdd(&stat[2], n_node * nval);
+            atomicAdd(&y.stat[0], n_int * nval);
+            atomicAdd(&y.stat[1], n_test);
+            atomicAdd(&y.stat[2], n_node * nval);
         }
     }
-    group_finish<ESTIMATE>(add2(anx, alx), add2(any, aly), v0, v1, i0, i1, p0, p1, vel_in, pos_out, vel_out, acc_rec,
-                           k, hdt, amag, ext);
+    return true;
+}
+
+// The lists of one slot on the lane's two particles.
+template <bool EXACT, bool QUAD, class SM>
+__device__ __forceinline__ void sum_slot(const GroupSys& y, SM& g, const typename SM::Slot& sl, uint32_t nodes,
+                                         uint32_t runs, float2 P, float2 Q, float2 E2, float2& anx, float2& any,
+                                         float2& alx, float2& aly, int lane) {
+    eval_nodes<EXACT, QUAD>(sl.node, g.ca, g.cb, nodes, y.rec, y.quad, P, Q, E2, anx, any, lane);
+    eval_leaves<EXACT, SM::kItem>(sl.run, g.off, g.ca, runs, y.rec, P, Q, E2, alx, aly, lane);
+}
+
+// One group, on one warp or (SPLIT) two: `walker` says which of the two this is, `phase` holds
+// this warp's phases of the slots' barriers.  False if a wait on the other warp ran out.
+// ESTIMATE: the |a| estimate pass of the relative criterion.  A group whose particles all
+// have a previous |a| returns at once; any other group walks with the theta test and
+// writes only the |a| of its particles (no integration), which the following normal pass
+// then opens nodes by.
+template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, class SM>
+__device__ __forceinline__ bool force_group_body(const GroupSys& y, uint32_t group, bool walker, uint32_t& phase, SM& g) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t nv = y.counts[0];
+    const uint32_t T = min(nv + y.counts[1], y.cap);
+    const uint32_t g0 = group * kGroupSize;
+    if (g0 >= nv || T == 0) return true;
+    if (ESTIMATE && !y.amag) return true;  // a batch member without the relative criterion
+    if (y.heavy && y.heavy[group]) return true;  // a costly group: walked by a warp pair (force_pair_body)
+    // particles: slot g0 + lane (.x of every pair) and g0 + 32 + lane (.y)
+    const uint32_t s0 = g0 + lane, s1 = s0 + 32;
+    const uint32_t i0 = s0 < nv ? y.sidx[s0] : 0u, i1 = s1 < nv ? y.sidx[s1] : 0u;
+    const bool v0 = s0 < nv && i0 < y.n_al, v1 = s1 < nv && i1 < y.n_al;  // i < n_al unless the sort failed
+    const float2 p0 = v0 ? y.pos_in[i0] : make_float2(0.0f, 0.0f);
+    const float2 p1 = v1 ? y.pos_in[i1] : make_float2(0.0f, 0.0f);
+    bool unknown = false;
+    float a0 = INFINITY, a1 = INFINITY;
+    if (y.amag && (walker || ESTIMATE)) {  // |a| is rewritten only after the walk
+        a0 = v0 ? y.amag[i0] : INFINITY;
+        a1 = v1 ? y.amag[i1] : INFINITY;
+        unknown = __any_sync(0xffffffffu, isnan(a0) || isnan(a1));
+        if (ESTIMATE && !unknown) return true;  // the same in both warps: nothing to estimate
+    }
+    const float2 P = make_float2(p0.x, p1.x), Q = make_float2(p0.y, p1.y), E2 = make_float2(y.eps2, y.eps2);
+    // node and leaf accumulators of the two particles (.x particle 0, .y particle 1)
+    float2 anx = make_float2(0.0f, 0.0f), any = anx, alx = anx, aly = anx;
+    bool ok = true;
+    if (!SM::kSplit) {
+        group_walk<COUNT, ESTIMATE>(y, g, nv, g0, s0, s1, v0, v1, p0, p1, unknown, a0, a1, lane,
+                                    [&](uint32_t, uint32_t nodes, uint32_t runs, bool) {
+                                        sum_slot<EXACT, QUAD>(y, g, g.slot[0], nodes, runs, P, Q, E2, anx, any, alx,
+                                                              aly, lane);
+                                        __syncwarp();  // the lists have been read
+                                        return true;
+                                    });
+    } else if (walker) {
+        uint32_t passed = 0;
+        ok = group_walk<COUNT, ESTIMATE>(y, g, nv, g0, s0, s1, v0, v1, p0, p1, unknown, a0, a1, lane,
+                                         [&](uint32_t b, uint32_t nodes, uint32_t runs, bool done) {
+                                             if (lane == 0) {
+                                                 g.slot[b].nodes = nodes;
+                                                 g.slot[b].runs = runs;
+                                                 g.slot[b].last = done ? 1u : 0u;
+                                             }
+                                             bar_pass(g.full[b], lane);
+                                             if (passed++) {  // the other slot's lists are summed
+                                                 if (!bar_wait(g.empty[b ^ 1u], phase >> (b ^ 1u) & 1u)) return false;
+                                                 phase ^= 1u << (b ^ 1u);
+                                             }
+                                             if (done) {  // and the last: the memory is free for the next group
+                                                 if (!bar_wait(g.empty[b], phase >> b & 1u)) return false;
+                                                 phase ^= 1u << b;
+                                             }
+                                             return true;
+                                         });
+    } else {
+        for (uint32_t b = 0, last = 0; !last; b ^= 1u) {
+            ok = bar_wait(g.full[b], phase >> b & 1u);
+            if (!ok) break;
+            phase ^= 1u << b;
+            const typename SM::Slot& sl = g.slot[b];
+            last = sl.last;
+            sum_slot<EXACT, QUAD>(y, g, sl, sl.nodes, sl.runs, P, Q, E2, anx, any, alx, aly, lane);
+            bar_pass(g.empty[b], lane);
+        }
+    }
+    if (!ok) {
+        if (lane == 0) atomicOr(y.err, kErrBarrierWait);
+        return false;
+    }
+    if (!SM::kSplit || !walker)
+        group_finish<ESTIMATE>(add2(anx, alx), add2(any, aly), v0, v1, i0, i1, p0, p1, y.vel_in, y.pos_out, y.vel_out,
+                               y.acc_rec, y.k, y.hdt, y.amag, y.ext);
+    return true;
 }
 
 // ------------------------------------------------------------------------------------
@@ -677,29 +845,24 @@ __device__ __forceinline__ void force_group_body(
 // only the summation order differs, and the CPU restatement follows it.
 // ------------------------------------------------------------------------------------
 // 64-record pops push at most 256 children, one level deeper than the shallowest popped
-// record: <= 192 D + 256 entries.
+// record: <= 192 D + 256 entries, the bottom of a deep stack in warp 0's local memory.
 constexpr int kPairStackCap = 192 * (kBBoxMaxBits > kFixedDepth ? kBBoxMaxBits : kFixedDepth) + 256;
-constexpr int kPairNode = 192, kPairItem = 256;  // a round adds <= 64 nodes and <= 128 runs
+constexpr int kPairNode = 128, kPairItem = 192;  // a round adds <= 64 nodes and <= 128 runs
 
-// No larger than the two single-warp walks it shares a block's shared memory with (the
-// traversal is sensitive to the L1 that shared memory leaves).
 struct PairSmem {
-    uint32_t stack[kPairStackCap];
+    uint32_t stack[kPairStackWindow];
     uint32_t node[kPairNode];
-    uint32_t it_start[kPairItem], it_count[kPairItem], off[kPairItem];
+    uint2 run[kPairItem];
+    uint32_t off[kPairItem];
     union {
         struct {
-            float cx[2][32], cy[2][32], cm[2][32];  // one staged chunk per warp
-            float qxx[2][32], qxy[2][32], qyy[2][32], mt[2][32];
+            float4 ca[2][32], cb[2][32];  // one staged chunk per warp
         };
         float2 part[4][32];  // after the sums: warp 1's accumulators, added by warp 0
     };
     uint32_t tot[2];  // packed round counts of each warp
+    uint32_t ticket;
 };
-static_assert(sizeof(PairSmem) <= 2 * sizeof(GroupSmem<160, 128>), "a pair walk fits in two warp walks");
-
-// Barrier of the two warps of pair `pair` (named barrier 1 + pair; __syncthreads uses 0).
-__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory"); }
 
 // Warp wp's share of the count accepted nodes in g.node, whose global list indices are
 // gbase .. gbase + count - 1: the 32-item chunks c with c mod 2 == wp, in order (each
@@ -722,15 +885,8 @@ __device__ __forceinline__ void pair_eval_nodes(PairSmem& g, int wp, uint32_t co
         }
     }
     for (; c * 32 < end; c += 2) {
-        g.cx[wp][lane] = q.x;
-        g.cy[wp][lane] = q.y;
-        g.cm[wp][lane] = q.z;
-        if (QUAD) {
-            g.qxx[wp][lane] = 7.5f * qq.x;
-            g.qxy[wp][lane] = 7.5f * qq.y;
-            g.qyy[wp][lane] = 7.5f * qq.z;
-            g.mt[wp][lane] = -1.5f * (qq.x + qq.z);
-        }
+        __syncwarp();
+        stage_node<QUAD>(g.ca[wp], g.cb[wp], lane, q, qq);
         __syncwarp();
         const uint32_t fn = (c + 2) * 32 + (uint32_t)lane;  // the warp's next chunk (all past gbase)
         if (fn < end) {
@@ -738,18 +894,10 @@ __device__ __forceinline__ void pair_eval_nodes(PairSmem& g, int wp, uint32_t co
             q = __ldg(&rec[r]);
             if (QUAD) qq = __ldg(&quad[r]);
         }
-        const uint32_t klo = gbase > c * 32 ? gbase - c * 32 : 0u;
-        const uint32_t khi = min(end - c * 32, 32u);
-#pragma unroll 4
-        for (uint32_t j = klo; j < khi; ++j) {
-            if (QUAD)
-                quadrupole_x2<EXACT>(g.cx[wp][j], g.cy[wp][j], g.cm[wp][j], g.qxx[wp][j], g.qxy[wp][j], g.qyy[wp][j],
-                                     g.mt[wp][j], P, Q, E2, acx, acy);
-            else
-                monopole_x2<EXACT>(g.cx[wp][j], g.cy[wp][j], g.cm[wp][j], P, Q, E2, acx, acy);
-        }
-        __syncwarp();
+        sum_chunk<EXACT, QUAD>(g.ca[wp], g.cb[wp], gbase > c * 32 ? gbase - c * 32 : 0u, min(end - c * 32, 32u), P, Q,
+                               E2, acx, acy);
     }
+    __syncwarp();
 }
 
 // Record fl of the flattened leaf runs of a pair (last run with off <= fl).
@@ -761,7 +909,7 @@ __device__ __forceinline__ float4 pair_gather_leaf(const PairSmem& g, uint32_t n
         if (g.off[mid] <= fl) lo = mid;
         else hi = mid - 1;
     }
-    return __ldg(&rec[g.it_start[lo] + (fl - g.off[lo])]);
+    return __ldg(&rec[g.run[lo].x + (fl - g.off[lo])]);
 }
 
 // Warp wp's share of the particle leaves of the n_items runs, whose flattened records have
@@ -772,29 +920,10 @@ __device__ __forceinline__ uint32_t pair_eval_leaves(PairSmem& g, int pair, int 
                                                      const float4* __restrict__ rec, float2 P, float2 Q, float2 E2,
                                                      float2& acx, float2& acy, int lane) {
     if (!n_items) return 0u;
-    constexpr int kPer = kPairItem / 32;
-    uint32_t cnt[kPer], sum = 0;
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-        const uint32_t it = (uint32_t)lane * kPer + t;
-        cnt[t] = it < n_items ? g.it_count[it] : 0u;
-        sum += cnt[t];
-    }
-    uint32_t x = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
-    if (wp == 0) {
-        uint32_t run = x - sum;
-#pragma unroll
-        for (int t = 0; t < kPer; ++t) {
-            g.off[lane * kPer + t] = run;
-            run += cnt[t];
-        }
-    }
+    uint32_t total = 0;
+    if (wp == 0) total = run_offsets<kPairItem / 32>(g.run, g.off, n_items, lane);
     pair_sync(pair);
+    total = g.off[n_items - 1] + g.run[n_items - 1].y;
     const uint32_t end = lbase + total;
     uint32_t c = lbase >> 5;
     if ((c & 1u) != (uint32_t)wp) ++c;
@@ -805,18 +934,15 @@ __device__ __forceinline__ uint32_t pair_eval_leaves(PairSmem& g, int pair, int 
         if (f >= lbase && f < end) q = pair_gather_leaf(g, n_items, f - lbase, rec);
     }
     for (; c * 32 < end; c += 2) {
-        g.cx[wp][lane] = q.x;
-        g.cy[wp][lane] = q.y;
-        g.cm[wp][lane] = q.z;
+        __syncwarp();
+        g.ca[wp][lane] = q;
         __syncwarp();
         const uint32_t fn = (c + 2) * 32 + (uint32_t)lane;
         if (fn < end) q = pair_gather_leaf(g, n_items, fn - lbase, rec);
-        const uint32_t klo = lbase > c * 32 ? lbase - c * 32 : 0u;
-        const uint32_t khi = min(end - c * 32, 32u);
-#pragma unroll 4
-        for (uint32_t j = klo; j < khi; ++j) monopole_x2<EXACT>(g.cx[wp][j], g.cy[wp][j], g.cm[wp][j], P, Q, E2, acx, acy);
-        __syncwarp();
+        sum_chunk<EXACT, false>(g.ca[wp], nullptr, lbase > c * 32 ? lbase - c * 32 : 0u, min(end - c * 32, 32u), P, Q,
+                                E2, acx, acy);
     }
+    __syncwarp();
     return total;
 }
 
@@ -824,36 +950,30 @@ __device__ __forceinline__ uint32_t pair_eval_leaves(PairSmem& g, int pair, int 
 // with the same arguments.  Warp 0 integrates.
 template <bool EXACT, bool COUNT>
 __device__ __forceinline__ void force_pair_body(
-    uint32_t group, int pair, int wp, PairSmem& g, const uint32_t* __restrict__ sidx,
-    const uint32_t* __restrict__ skey, const uint32_t* __restrict__ counts, const float4* __restrict__ rec,
-    const uint32_t* __restrict__ skip, const float4* __restrict__ quad, const uint4* __restrict__ kids,
-    const float2* __restrict__ pos_in, const float2* __restrict__ vel_in, float2* __restrict__ pos_out,
-    float2* __restrict__ vel_out, float2* __restrict__ acc_rec, uint32_t n_al, float eps2, float k, float hdt,
-    uint32_t cap, unsigned long long* __restrict__ stat, int* __restrict__ err, float* __restrict__ amag,
-    float alpha, float floor2, uint32_t* __restrict__ ext) {
+    const GroupSys& y, uint32_t group, int pair, int wp, PairSmem& g) {
     const int lane = threadIdx.x & 31;
-    const uint32_t nv = counts[0];
-    const uint32_t T = min(nv + counts[1], cap);
+    const uint32_t nv = y.counts[0];
+    const uint32_t T = min(nv + y.counts[1], y.cap);
     const uint32_t g0 = group * kGroupSize;
     if (g0 >= nv || T == 0) return;  // never for a listed group; the same for both warps
     const uint32_t s0 = g0 + lane, s1 = s0 + 32;
-    const uint32_t i0 = s0 < nv ? sidx[s0] : 0u, i1 = s1 < nv ? sidx[s1] : 0u;
-    const bool v0 = s0 < nv && i0 < n_al, v1 = s1 < nv && i1 < n_al;
-    const float2 p0 = v0 ? pos_in[i0] : make_float2(0.0f, 0.0f);
-    const float2 p1 = v1 ? pos_in[i1] : make_float2(0.0f, 0.0f);
+    const uint32_t i0 = s0 < nv ? y.sidx[s0] : 0u, i1 = s1 < nv ? y.sidx[s1] : 0u;
+    const bool v0 = s0 < nv && i0 < y.n_al, v1 = s1 < nv && i1 < y.n_al;
+    const float2 p0 = v0 ? y.pos_in[i0] : make_float2(0.0f, 0.0f);
+    const float2 p1 = v1 ? y.pos_in[i1] : make_float2(0.0f, 0.0f);
     float bx0[4], bx1[4], by0[4], by1[4];
-    group_boxes(skey, g0, nv, s0, s1, v0, v1, p0, p1, bx0, bx1, by0, by1);
-    float amin = fminf(v0 ? amag[i0] : INFINITY, v1 ? amag[i1] : INFINITY);  // every |a| is known
+    group_boxes(y.skey, g0, nv, s0, s1, v0, v1, p0, p1, bx0, bx1, by0, by1);
+    float amin = fminf(v0 ? y.amag[i0] : INFINITY, v1 ? y.amag[i1] : INFINITY);  // every |a| is known
     for (int o = 16; o; o >>= 1) amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
-    const float tol = alpha * amin, tol2 = tol * tol;
-    const float2 P = make_float2(p0.x, p1.x), Q = make_float2(p0.y, p1.y), E2 = make_float2(eps2, eps2);
+    const float tol = y.alpha * amin, tol2 = tol * tol;
+    const float2 P = make_float2(p0.x, p1.x), Q = make_float2(p0.y, p1.y), E2 = make_float2(y.eps2, y.eps2);
     float2 anx = make_float2(0.0f, 0.0f), any = anx, alx = anx, aly = anx;
     unsigned long long n_int = 0, n_test = 0, n_node = 0;
+    StackSpill<kPairStackCap, kPairStackSpill> spill;
     uint32_t size = 0, n_nodes = 0, n_items = 0, gnode = 0, gleaf = 0;
-    if (skip[0] == 1u) {  // a single particle: the root is its leaf
+    if (y.skip[0] == 1u) {  // a single particle: the root is its leaf
         if (wp == 0 && lane == 0) {
-            g.it_start[0] = 0u;
-            g.it_count[0] = 1u;
+            g.run[0] = make_uint2(0u, 1u);
         }
         n_items = 1;
     } else {
@@ -862,16 +982,21 @@ __device__ __forceinline__ void force_pair_body(
     }
     for (;;) {
         pair_sync(pair);  // the last round's lists, pushes and counts are visible
-        if (size == 0) break;
+        if (size == 0 && spill.count == 0) break;
         if (n_nodes > (uint32_t)(kPairNode - 64)) {
-            pair_eval_nodes<EXACT, true>(g, wp, n_nodes, gnode, rec, quad, P, Q, E2, anx, any, lane);
+            pair_eval_nodes<EXACT, true>(g, wp, n_nodes, gnode, y.rec, y.quad, P, Q, E2, anx, any, lane);
             gnode += n_nodes;
             n_nodes = 0;
             pair_sync(pair);
         }
         if (n_items > (uint32_t)(kPairItem - 128)) {
-            gleaf += pair_eval_leaves<EXACT>(g, pair, wp, n_items, gleaf, rec, P, Q, E2, alx, aly, lane);
+            gleaf += pair_eval_leaves<EXACT>(g, pair, wp, n_items, gleaf, y.rec, P, Q, E2, alx, aly, lane);
             n_items = 0;
+            pair_sync(pair);
+        }
+        if (size < 64u && spill.count) {  // the same in both warps; warp 0 holds the entries
+            if (wp == 0) size = spill.restore(g.stack, size, lane);
+            else size += kPairStackSpill, spill.count -= kPairStackSpill;
             pair_sync(pair);
         }
         const uint32_t np = min(size, 64u);
@@ -883,7 +1008,7 @@ __device__ __forceinline__ void force_pair_body(
         size = base;
         if (COUNT) n_test += __popc(__ballot_sync(0xffffffffu, act));
         RecTest r{};
-        if (act) test_record(n, rec, kids, bx0, bx1, by0, by1, eps2, true, tol2, floor2, 0.0f, r);
+        if (act) test_record(n, y.rec, y.kids, bx0, bx1, by0, by1, y.eps2, true, tol2, y.floor2, 0.0f, r);
         // offsets in pair order: this warp's scan plus warp 0's total for warp 1; nodes
         // <= 64, runs <= 128 and pushes <= 256 in pair total, so the 8/8/16-bit fields
         // never carry
@@ -900,20 +1025,19 @@ __device__ __forceinline__ void force_pair_body(
         const uint32_t noff = ex & 0xffu, loff = (ex >> 8) & 0xffu, poff = ex >> 16;
         const uint32_t ntot = tot & 0xffu, ltot = (tot >> 8) & 0xffu;
         uint32_t ptot = tot >> 16, npu = r.npu;
-        if (size + ptot > (uint32_t)kPairStackCap) {  // beyond the depth bound: report, do not overrun
-            if (wp == 0 && lane == 0) atomicOr(err, kErrTree);
+        if (size + ptot > (uint32_t)kPairStackWindow) {
+            if (wp == 0) size = spill.save(g.stack, size, lane);
+            else size -= kPairStackSpill, spill.count += kPairStackSpill;
+            pair_sync(pair);
+        }
+        if (spill.count + size + ptot > (uint32_t)kPairStackCap) {  // beyond the depth bound: report, do not overrun
+            if (wp == 0 && lane == 0) atomicOr(y.err, kErrTree);
             ptot = 0;
             npu = 0;
         }
         if (r.nn) g.node[n_nodes + noff] = n;
-        if (r.nl > 0) {
-            g.it_start[n_items + loff] = r.a0;
-            g.it_count[n_items + loff] = r.c0;
-        }
-        if (r.nl > 1) {
-            g.it_start[n_items + loff + 1] = r.a1;
-            g.it_count[n_items + loff + 1] = r.c1;
-        }
+        if (r.nl > 0) g.run[n_items + loff] = make_uint2(r.a0, r.c0);
+        if (r.nl > 1) g.run[n_items + loff + 1] = make_uint2(r.a1, r.c1);
         if (COUNT) {
             n_int += r.nn + (r.nl > 0 ? r.c0 : 0u) + (r.nl > 1 ? r.c1 : 0u);
             n_node += r.nn;
@@ -927,19 +1051,19 @@ __device__ __forceinline__ void force_pair_body(
         n_items += ltot;
         size += ptot;
     }
-    pair_eval_nodes<EXACT, true>(g, wp, n_nodes, gnode, rec, quad, P, Q, E2, anx, any, lane);
-    pair_eval_leaves<EXACT>(g, pair, wp, n_items, gleaf, rec, P, Q, E2, alx, aly, lane);
+    pair_eval_nodes<EXACT, true>(g, wp, n_nodes, gnode, y.rec, y.quad, P, Q, E2, anx, any, lane);
+    pair_eval_leaves<EXACT>(g, pair, wp, n_items, gleaf, y.rec, P, Q, E2, alx, aly, lane);
     if (COUNT) {
-        if (skip[0] == 1u && wp == 0 && lane == 0) n_int += 1;
+        if (y.skip[0] == 1u && wp == 0 && lane == 0) n_int += 1;
         for (int o = 16; o; o >>= 1) {
             n_int += __shfl_xor_sync(0xffffffffu, n_int, o);
             n_node += __shfl_xor_sync(0xffffffffu, n_node, o);
         }
         const unsigned long long nval = __popc(__ballot_sync(0xffffffffu, v0)) + __popc(__ballot_sync(0xffffffffu, v1));
         if (lane == 0) {
-            atomicAdd(&stat[0], n_int * nval);
-            atomicAdd(&stat[1], n_test);
-            atomicAdd(&stat[2], n_node * nval);
+            atomicAdd(&y.stat[0], n_int * nval);
+            atomicAdd(&y.stat[1], n_test);
+            atomicAdd(&y.stat[2], n_node * nval);
         }
     }
     pair_sync(pair);  // both warps are done with their staged chunks
@@ -955,119 +1079,137 @@ __device__ __forceinline__ void force_pair_body(
         any = add2(any, g.part[1][lane]);
         alx = add2(alx, g.part[2][lane]);
         aly = add2(aly, g.part[3][lane]);
-        group_finish<false>(add2(anx, alx), add2(any, aly), v0, v1, i0, i1, p0, p1, vel_in, pos_out, vel_out,
-                            acc_rec, k, hdt, amag, ext);
+        group_finish<false>(add2(anx, alx), add2(any, aly), v0, v1, i0, i1, p0, p1, y.vel_in, y.pos_out,
+                            y.vel_out, y.acc_rec, y.k, y.hdt, y.amag, y.ext);
     }
     pair_sync(pair);  // the pair's shared memory is free for its next group
 }
 
-// list caps of a shape
-template <bool SHORT>
-using GroupSmemOf = GroupSmem<SHORT ? 96 : 160, SHORT ? 64 : 128>;
-
-// Shared memory of a traversal block: a walk per warp, and with HEAVY (the main pass of
-// the relative criterion) the bytes of warps 2p and 2p + 1 also hold the walk of warp pair
-// p, so that a pair done with costly groups starts its own warps' walks at once.
-template <bool SHORT, int WARPS, bool HEAVY>
-struct ForceSmem {
-    GroupSmemOf<SHORT> warp[WARPS];
-    __device__ __forceinline__ GroupSmemOf<SHORT>& walk(int w) { return warp[w]; }
-};
-template <bool SHORT>
-union PairSlot {
-    GroupSmemOf<SHORT> warp[2];
-    PairSmem pair;
-};
-template <bool SHORT, int WARPS>
-struct ForceSmem<SHORT, WARPS, true> {
-    PairSlot<SHORT> slot[WARPS / 2];
-    __device__ __forceinline__ GroupSmemOf<SHORT>& walk(int w) { return slot[w >> 1].warp[w & 1]; }
+// The launch of a group-walk kernel: GROUPS groups per block, on one warp each or (SPLIT) two;
+// long or short lists (gs_shape).
+template <int GROUPS, bool SHORT, bool SPLIT>
+struct WalkShape {
+    using Smem = typename std::conditional<SPLIT, GroupSmem<SHORT ? 31 : 63, SHORT ? 31 : 63, 2>,
+                                           GroupSmem<SHORT ? 64 : 128, SHORT ? 32 : 64, 1>>::type;
+    static constexpr int kGroups = GROUPS, kThreads = GROUPS * (SPLIT ? 64 : 32);
+    // resident blocks the registers are cut for: one warp per group at 96 registers a thread
+    // (20 groups an SM), two at 128 (8 groups: N = 100,000, 161 us a step against 167 with 12 and 179 with 16)
+    static constexpr int kBlocks = (SPLIT ? kSplitPerSm : kSinglePerSm) / GROUPS;
+    static constexpr bool kSplit = SPLIT;
 };
 
-// The next listed costly group for warp pair `pair` (hwork[0] entries, hwork[1] the next
-// to take), or a value >= hwork[0] when none is left.  Both warps of the pair call it.
-__device__ __forceinline__ uint32_t pair_ticket(uint32_t* __restrict__ hwork, uint32_t cnt, uint32_t* s_u, int pair) {
-    if ((threadIdx.x & 63u) == 0) s_u[pair] = __ldcg(&hwork[1]) < cnt ? atomicAdd(&hwork[1], 1u) : cnt;
+// Shared memory of a block; with HEAVY (the main pass of the relative criterion) each pair of
+// warps first walks costly groups together in the bytes of its one (SPLIT) or two groups.
+template <class SH, bool HEAVY>
+struct WalkSmem {
+    typename SH::Smem g[SH::kGroups];
+    uint32_t ticket[SH::kThreads / 32];
+    __device__ __forceinline__ typename SH::Smem& walk(int i) { return g[i]; }
+};
+template <class SH>
+struct WalkSmem<SH, true> {
+    static constexpr int kPer = SH::kSplit ? 1 : 2;  // groups per pair of warps
+    union Pair {
+        typename SH::Smem g[kPer];
+        PairSmem pair;
+    } p[SH::kThreads / 64];
+    uint32_t ticket[SH::kThreads / 32];
+    __device__ __forceinline__ typename SH::Smem& walk(int i) { return p[i / kPer].g[i % kPer]; }
+};
+
+// The next value of a counter below cnt for both warps of a pair, or a value >= cnt when none
+// is left.
+__device__ __forceinline__ uint32_t pair_ticket(uint32_t* __restrict__ next, uint32_t cnt, uint32_t& s_u, int pair) {
+    if ((threadIdx.x & 63u) == 0) s_u = __ldcg(next) < cnt ? atomicAdd(next, 1u) : cnt;
     pair_sync(pair);
-    const uint32_t u = s_u[pair];
-    pair_sync(pair);  // read by both warps before the pair's next ticket
+    const uint32_t u = s_u;
+    pair_sync(pair);  // read by both warps before the next ticket
     return u;
 }
-
-// With HEAVY every warp pair first walks listed costly groups (heavy_list[u].y, taken in
-// order from hwork) and then each warp its own group: the costly walks start first.
-template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, int WARPS, bool SHORT, bool HEAVY>
-__global__ void __launch_bounds__(WARPS * 32)
-k_force_group(const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ counts,
-              const float4* __restrict__ rec, const uint32_t* __restrict__ skip, const float4* __restrict__ quad,
-              const uint4* __restrict__ kids, const float2* __restrict__ pos_in, const float2* __restrict__ vel_in,
-              float2* __restrict__ pos_out, float2* __restrict__ vel_out, float2* __restrict__ acc_rec,
-              uint32_t n_al, float eps2, float theta2, float k, float hdt, uint32_t cap,
-              unsigned long long* __restrict__ stat, int* __restrict__ err, float* __restrict__ amag, float alpha,
-              float floor2, uint32_t* __restrict__ ext, const uint8_t* __restrict__ heavy,
-              const uint2* __restrict__ heavy_list, uint32_t* __restrict__ hwork) {
-    pdl_enter();
-    __shared__ ForceSmem<SHORT, WARPS, HEAVY> sm;
-    if constexpr (HEAVY) {
-        static_assert(QUAD && !ESTIMATE && WARPS % 2 == 0, "warp pairs walk costly groups of the relative main pass");
-        __shared__ uint32_t s_u[WARPS / 2];
-        const int pair = (int)(threadIdx.x >> 6), wp = (int)((threadIdx.x >> 5) & 1u);
-        const uint32_t cnt = hwork[0];
-        for (uint32_t u; (u = pair_ticket(hwork, cnt, s_u, pair)) < cnt;)
-            force_pair_body<EXACT, COUNT>(heavy_list[u].y, pair, wp, sm.slot[pair].pair, sidx, skey, counts, rec, skip,
-                                          quad, kids, pos_in, vel_in, pos_out, vel_out, acc_rec, n_al, eps2, k, hdt,
-                                          cap, stat, err, amag, alpha, floor2, ext);
-    }
-    force_group_body<EXACT, QUAD, COUNT, ESTIMATE, WARPS>(grid_blk(), sm.walk((int)(threadIdx.x >> 5)), sidx, skey,
-                                                   counts, rec, skip, quad, kids, pos_in, vel_in, pos_out, vel_out,
-                                                   acc_rec, n_al, eps2, theta2, k, hdt, cap, stat, err, amag, alpha,
-                                                   floor2, ext, HEAVY ? heavy : nullptr);
+// The same for one warp.
+__device__ __forceinline__ uint32_t warp_ticket(uint32_t* __restrict__ next, uint32_t cnt) {
+    uint32_t u = 0;
+    if ((threadIdx.x & 31u) == 0) u = __ldcg(next) < cnt ? atomicAdd(next, 1u) : cnt;
+    return __shfl_sync(0xffffffffu, u, 0);
 }
 
-// Batched: a persistent grid; with HEAVY each warp pair first takes costly groups
-// {member, group} from the batch's list, then every block takes block units of the
-// members from `work`.
-template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, int WARPS, bool SHORT, bool HEAVY>
-__global__ void __launch_bounds__(WARPS * 32)
+template <class SM>
+__device__ __forceinline__ void walk_init(SM& g, int pair) {
+    if (!SM::kSplit) return;
+    if ((threadIdx.x & 63u) < 2u) {
+        bar_init(g.full[threadIdx.x & 1u]);
+        bar_init(g.empty[threadIdx.x & 1u]);
+    }
+    pair_sync(pair);
+}
+
+// Which of a walk's two warps walks: alternating over walks and blocks, so that the summing
+// warps, which keep the FMA pipe busy, spread over the four schedulers.
+__device__ __forceinline__ bool is_walker() {
+    const uint32_t warp = threadIdx.x >> 5;
+    return ((warp + (warp >> 1) + blockIdx.x) & 1u) == 0;
+}
+
+// With HEAVY every pair of warps first takes listed costly groups (heavy_list[u].y, in order
+// from hwork) and then its own: the costly walks start first.
+template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, class SH, bool HEAVY>
+__global__ void __launch_bounds__(SH::kThreads, SH::kBlocks)
+k_force_group(GroupSys y, const uint2* __restrict__ heavy_list, uint32_t* __restrict__ hwork) {
+    __shared__ __align__(16) WalkSmem<SH, HEAVY> sm;
+    pdl_enter();
+    const int pair = (int)(threadIdx.x >> 6), walk = SH::kSplit ? pair : (int)(threadIdx.x >> 5);
+    if constexpr (HEAVY) {
+        static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
+        const uint32_t cnt = hwork[0];
+        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.ticket[pair], pair)) < cnt;)
+            force_pair_body<EXACT, COUNT>(y, heavy_list[u].y, pair, (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
+    }
+    walk_init(sm.walk(walk), pair);
+    uint32_t phase = 0;
+    force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(y, blockIdx.x * SH::kGroups + walk, !SH::kSplit || is_walker(), phase,
+                                                   sm.walk(walk));
+}
+
+__device__ __forceinline__ GroupSys batch_group_sys(const SysDesc& d, int in, int out, bool heavy) {
+    const int f = d.passes & 1;
+    return GroupSys{d.idx[f], d.keys[f], d.counters + kCtrValid, d.rec, d.skip, d.quad, d.kids, d.pos[in], d.vel[in],
+                    d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.theta2, d.k, d.hdt, d.cap,
+                    (unsigned long long*)(d.counters + kCtrStat), d.err, d.amag, d.alpha, d.floor2,
+                    d.ext ? d.ext + 4 * out : nullptr, heavy ? d.heavy : nullptr};
+}
+
+// Batched: a persistent grid; with HEAVY each pair of warps first takes costly groups
+// {member, group} from the batch's list, then every walk takes groups of the members from
+// `work`.
+template <bool EXACT, bool QUAD, bool COUNT, bool ESTIMATE, class SH, bool HEAVY>
+__global__ void __launch_bounds__(SH::kThreads, SH::kBlocks)
 kb_force_group(BatchArgs a, uint32_t* __restrict__ work, const uint2* __restrict__ heavy_list,
                uint32_t* __restrict__ hwork) {
+    __shared__ __align__(16) WalkSmem<SH, HEAVY> sm;
     pdl_enter();
-    __shared__ ForceSmem<SHORT, WARPS, HEAVY> sm;
-    __shared__ uint32_t s_b;
+    const int pair = (int)(threadIdx.x >> 6), walk = SH::kSplit ? pair : (int)(threadIdx.x >> 5);
     if constexpr (HEAVY) {
-        static_assert(QUAD && !ESTIMATE && WARPS % 2 == 0, "warp pairs walk costly groups of the relative main pass");
-        __shared__ uint32_t s_u[WARPS / 2];
-        const int pair = (int)(threadIdx.x >> 6), wp = (int)((threadIdx.x >> 5) & 1u);
+        static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
         const uint32_t cnt = hwork[0];
-        for (uint32_t u; (u = pair_ticket(hwork, cnt, s_u, pair)) < cnt;) {
+        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.ticket[pair], pair)) < cnt;) {
             const uint2 e = heavy_list[u];
             const SysDesc& d = a.descs[e.x];
-            const int in = (int)((d.parity + a.step) & 1u), out = in ^ 1;
-            const int f = d.passes & 1;
-            force_pair_body<EXACT, COUNT>(e.y, pair, wp, sm.slot[pair].pair, d.idx[f], d.keys[f],
-                                          d.counters + kCtrValid, d.rec, d.skip, d.quad, d.kids, d.pos[in],
-                                          d.vel[in], d.pos[out], d.vel[out], d.acc, d.n_al, d.eps2, d.k, d.hdt,
-                                          d.cap, (unsigned long long*)(d.counters + kCtrStat), d.err, d.amag,
-                                          d.alpha, d.floor2, d.ext ? d.ext + 4 * out : nullptr);
+            const int in = (int)((d.parity + a.step) & 1u);
+            force_pair_body<EXACT, COUNT>(batch_group_sys(d, in, in ^ 1, false), e.y, pair,
+                                          (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
         }
     }
+    walk_init(sm.walk(walk), pair);
     const uint32_t total = __ldg(&a.first[a.nsys]);
+    const bool walker = !SH::kSplit || is_walker();
+    uint32_t phase = 0;
     for (;;) {
-        __syncthreads();  // every thread has read the previous s_b
-        if (threadIdx.x == 0) s_b = atomicAdd(work, 1u);
-        __syncthreads();
-        const uint32_t b = s_b;
-        if (b >= total) break;
-        const BatchBlock bb = batch_block(a, b);
-        const SysDesc& d = *bb.d;
-        const int f = d.passes & 1;
-        force_group_body<EXACT, QUAD, COUNT, ESTIMATE, WARPS>(bb.blk, sm.walk((int)(threadIdx.x >> 5)), d.idx[f],
-                                             d.keys[f], d.counters + kCtrValid, d.rec, d.skip, d.quad, d.kids,
-                                             d.pos[bb.in], d.vel[bb.in], d.pos[bb.out], d.vel[bb.out], d.acc, d.n_al,
-                                             d.eps2, d.theta2, d.k, d.hdt, d.cap,
-                                             (unsigned long long*)(d.counters + kCtrStat), d.err, d.amag, d.alpha,
-                                             d.floor2, d.ext ? d.ext + 4 * bb.out : nullptr,
-                                             HEAVY ? d.heavy : nullptr);
+        const uint32_t u = SH::kSplit ? pair_ticket(work, total, sm.ticket[pair], pair) : warp_ticket(work, total);
+        if (u >= total) break;
+        const BatchBlock bb = batch_block(a, u);
+        if (!force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(batch_group_sys(*bb.d, bb.in, bb.out, HEAVY), bb.blk.id,
+                                                            walker, phase, sm.walk(walk)))
+            break;
     }
 }
 
@@ -1103,77 +1245,68 @@ __global__ void __launch_bounds__(kForceWarps * 32, 6) kb_force(BatchArgs a, uin
 namespace gsim {
 namespace {
 
-using GroupFn = void (*)(const uint32_t*, const uint32_t*, const uint32_t*, const float4*, const uint32_t*,
-                         const float4*, const uint4*, const float2*, const float2*, float2*, float2*, float2*,
-                         uint32_t, float, float, float, float, uint32_t, unsigned long long*, int*, float*, float,
-                         float, uint32_t*, const uint8_t*, const uint2*, uint32_t*);
+using GroupFn = void (*)(GroupSys, const uint2*, uint32_t*);
 using BatchGroupFn = void (*)(BatchArgs, uint32_t*, const uint2*, uint32_t*);
 
 // The group-walk kernel of one shape (counting variants: the default shape only); heavy:
-// the main pass with warp pairs for costly groups (quadrupoles, relative criterion).
-template <bool EXACT, int W, bool S>
+// the main pass with warp pairs for costly groups (quadrupoles, relative criterion), which
+// need two warps per block at least.
+template <bool EXACT, bool COUNT, class SH>
 GroupFn group_fn(bool quad, bool est, bool heavy) {
-    if (est) return k_force_group<EXACT, true, false, true, W, S, false>;
-    if constexpr (W % 2 == 0)
-        if (heavy) return k_force_group<EXACT, true, false, false, W, S, true>;
-    return quad ? k_force_group<EXACT, true, false, false, W, S, false>
-                : k_force_group<EXACT, false, false, false, W, S, false>;
+    if (est) return k_force_group<EXACT, true, COUNT, true, SH, false>;
+    if constexpr (SH::kThreads >= 64)
+        if (heavy) return k_force_group<EXACT, true, COUNT, false, SH, true>;
+    return quad ? k_force_group<EXACT, true, COUNT, false, SH, false>
+                : k_force_group<EXACT, false, COUNT, false, SH, false>;
 }
-template <bool EXACT>
-GroupFn group_fn_count(bool quad, bool est, bool heavy) {
-    if (est) return k_force_group<EXACT, true, true, true, 2, false, false>;
-    if (heavy) return k_force_group<EXACT, true, true, false, 2, false, true>;
-    return quad ? k_force_group<EXACT, true, true, false, 2, false, false>
-                : k_force_group<EXACT, false, true, false, 2, false, false>;
-}
-template <bool EXACT, int W, bool S>
+template <bool EXACT, bool COUNT, class SH>
 BatchGroupFn batch_group_fn(bool quad, bool est, bool heavy) {
-    if (est) return kb_force_group<EXACT, true, false, true, W, S, false>;
-    if constexpr (W % 2 == 0)
-        if (heavy) return kb_force_group<EXACT, true, false, false, W, S, true>;
-    return quad ? kb_force_group<EXACT, true, false, false, W, S, false>
-                : kb_force_group<EXACT, false, false, false, W, S, false>;
-}
-template <bool EXACT>
-BatchGroupFn batch_group_fn_count(bool quad, bool est, bool heavy) {
-    if (est) return kb_force_group<EXACT, true, true, true, 2, false, false>;
-    if (heavy) return kb_force_group<EXACT, true, true, false, 2, false, true>;
-    return quad ? kb_force_group<EXACT, true, true, false, 2, false, false>
-                : kb_force_group<EXACT, false, true, false, 2, false, false>;
+    if (est) return kb_force_group<EXACT, true, COUNT, true, SH, false>;
+    if constexpr (SH::kThreads >= 64)
+        if (heavy) return kb_force_group<EXACT, true, COUNT, false, SH, true>;
+    return quad ? kb_force_group<EXACT, true, COUNT, false, SH, false>
+                : kb_force_group<EXACT, false, COUNT, false, SH, false>;
 }
 
-// warps per block and list caps actually launched for a request (warp pairs need an even
-// number of warps: a one-warp shape runs with two when costly groups are paired)
-inline void group_shape(bool count, const gs_shape& sh, bool heavy, int* warps, bool* shrt) {
-    *warps = count ? 2 : (int)sh.force_warps;
-    if (heavy && *warps == 1) *warps = 2;
-    *shrt = count ? false : sh.force_short_lists != 0;
+// fn(shape) with the shape launched for a request, its groups and threads per block.
+template <class Fn>
+auto with_shape(bool count, const gs_shape& sh, bool split, bool heavy, int* groups, int* threads, Fn&& fn) {
+    const auto use = [&](auto shape) {
+        *groups = decltype(shape)::kGroups;
+        *threads = decltype(shape)::kThreads;
+        return fn(shape);
+    };
+    if (count) return use(WalkShape<2, false, false>{});
+    const uint32_t g = heavy && !split && sh.force_warps == 1 ? 2u : sh.force_warps;
+    if (sh.force_short_lists) return split ? use(WalkShape<2, true, true>{}) : use(WalkShape<2, true, false>{});
+    if (g == 1) return split ? use(WalkShape<1, false, true>{}) : use(WalkShape<1, false, false>{});
+    if (g == 4) return split ? use(WalkShape<4, false, true>{}) : use(WalkShape<4, false, false>{});
+    return split ? use(WalkShape<2, false, true>{}) : use(WalkShape<2, false, false>{});
+}
+
+// Two warps per group where the launch's groups cannot fill the SMs on one warp each.
+constexpr uint32_t kSplitGroups = 152 * 14;
+
+template <bool EXACT>
+GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad, bool est, bool heavy, int* groups,
+                   int* threads) {
+    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
+        using SH = decltype(s);
+        if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
+            if (count) return group_fn<EXACT, true, SH>(quad, est, heavy);
+        return group_fn<EXACT, false, SH>(quad, est, heavy);
+    });
 }
 
 template <bool EXACT>
-GroupFn pick_group(bool count, const gs_shape& sh, bool quad, bool est, bool heavy, int* warps) {
-    bool shrt;
-    group_shape(count, sh, heavy, warps, &shrt);
-    if (count) return group_fn_count<EXACT>(quad, est, heavy);
-    switch (*warps * 2 + (shrt ? 1 : 0)) {
-        case 2: return group_fn<EXACT, 1, false>(quad, est, false);
-        case 5: return group_fn<EXACT, 2, true>(quad, est, heavy);
-        case 8: return group_fn<EXACT, 4, false>(quad, est, heavy);
-        default: *warps = 2; return group_fn<EXACT, 2, false>(quad, est, heavy);
-    }
-}
-
-template <bool EXACT>
-BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, bool quad, bool est, bool heavy, int* warps) {
-    bool shrt;
-    group_shape(count, sh, heavy, warps, &shrt);
-    if (count) return batch_group_fn_count<EXACT>(quad, est, heavy);
-    switch (*warps * 2 + (shrt ? 1 : 0)) {
-        case 2: return batch_group_fn<EXACT, 1, false>(quad, est, false);
-        case 5: return batch_group_fn<EXACT, 2, true>(quad, est, heavy);
-        case 8: return batch_group_fn<EXACT, 4, false>(quad, est, heavy);
-        default: *warps = 2; return batch_group_fn<EXACT, 2, false>(quad, est, heavy);
-    }
+BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad, bool est, bool heavy,
+                              int* groups, int* threads) {
+    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
+        using SH = decltype(s);
+        if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
+            if (count) return batch_group_fn<EXACT, true, SH>(quad, est, heavy);
+        return batch_group_fn<EXACT, false, SH>(quad, est, heavy);
+    });
 }
 
 template <bool EXACT>
@@ -1196,14 +1329,16 @@ cudaError_t force_launch_impl(const ForceLaunch& f) {
         return launch(f.pdl, fn, blocks, kForceWarps * 32, f.st, f.sidx, f.counts, f.rec, f.skip, f.pos_in, f.vel_in,
                       f.pos_out, f.vel_out, f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
     }
-    int warps = 2;
+    int groups = 2, threads = 64;
     const bool heavy = f.heavy && f.quad && !f.estimate;
-    GroupFn fn = pick_group<EXACT>(f.count, f.shape, f.quad, f.estimate, heavy, &warps);
-    const int blocks = (int)((f.n_al / kGroupSize + warps - 1) / warps);
-    return launch(f.pdl, fn, blocks, warps * 32, f.st, f.sidx, f.skey, f.counts, f.rec, f.skip, f.quad_m, f.kids,
-                  f.pos_in, f.vel_in, f.pos_out, f.vel_out, f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap,
-                  f.stat, f.err, f.amag, f.alpha, f.floor2, f.ext, heavy ? f.heavy : nullptr,
-                  heavy ? f.heavy_list : nullptr, heavy ? f.heavy_work : nullptr);
+    const uint32_t n_groups = f.n_al / kGroupSize;
+    GroupFn fn = pick_group<EXACT>(f.count, f.shape, n_groups, f.quad, f.estimate, heavy, &groups, &threads);
+    const int blocks = (int)((n_groups + groups - 1) / groups);
+    const GroupSys y{f.sidx, f.skey, f.counts, f.rec, f.skip, f.quad_m, f.kids, f.pos_in, f.vel_in, f.pos_out, f.vel_out,
+                     f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.err, f.amag, f.alpha, f.floor2,
+                     f.ext, heavy ? f.heavy : nullptr};
+    return launch(f.pdl, fn, blocks, threads, f.st, y, heavy ? f.heavy_list : nullptr,
+                  heavy ? f.heavy_work : nullptr);
 }
 
 template <bool EXACT>
@@ -1223,11 +1358,11 @@ cudaError_t batch_force_launch_impl(const BatchForceLaunch& b, int* grid_out) {
         if (grid_out) return resident(fn);
         return launch(true, fn, b.grid, threads, b.st, BatchArgs{b.descs, b.first, b.nsys, b.step}, b.work);
     }
-    int warps = 2;
-    BatchGroupFn fn = pick_batch_group<EXACT>(b.count, b.shape, b.quad, b.estimate, heavy, &warps);
-    threads = warps * 32;
+    int groups = 2;
+    BatchGroupFn fn = pick_batch_group<EXACT>(b.count, b.shape, b.units, b.quad, b.estimate, heavy, &groups, &threads);
     if (grid_out) return resident(fn);
-    return launch(true, fn, b.grid, threads, b.st, BatchArgs{b.descs, b.first, b.nsys, b.step}, b.work,
+    const int grid = (int)(b.units + groups - 1) / groups;  // no more blocks than groups need
+    return launch(true, fn, b.grid < grid ? b.grid : grid, threads, b.st, BatchArgs{b.descs, b.first, b.nsys, b.step}, b.work,
                   heavy ? b.heavy_list : nullptr, heavy ? b.heavy_work : nullptr);
 }
 

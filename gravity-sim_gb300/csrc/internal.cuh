@@ -365,6 +365,7 @@ struct BatchForceLaunch {
     uint32_t nsys = 0, step = 0;
     uint32_t* work = nullptr;
     int grid = 0;
+    uint32_t units = 0;  // entries of the block table: groups (group walk) or blocks
     bool group = false, quad = false, count = false, estimate = false;
     gs_shape shape{};
     const uint2* heavy_list = nullptr;  // the batch's costly groups, or null
@@ -376,8 +377,7 @@ cudaError_t batch_force_launch_exact(const BatchForceLaunch& b, int* grid_out);
 bool force_shape_supported(uint32_t warps, uint32_t short_lists);
 
 // batched stages (one launch per stage over every system of a plan)
-// force_warps: group walks per block of the batch's traversal launch (its block table)
-void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& shape, uint32_t force_warps);
+void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& shape);
 void direct_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& batch_shape);
 // j-chunks the direct sum of `s` splits into under a shape (its scratch holds direct_max_chunks)
 uint32_t direct_chunks_needed(const gs_sim* s, const gs_shape& sh);
