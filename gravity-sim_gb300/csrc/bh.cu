@@ -23,8 +23,9 @@
 //   monopole mode (the reference's rule):
 //   k_coop_sums   mass and mass-moment sums level by level, finest first (one cooperative
 //                 launch, a grid barrier between deep levels, one block for the top
-//                 levels; a batch launches kb_level_sums per level), children in the order
-//                 of TreeInitShader.comp:78-80; centre of mass as TreeMoveShader.comp:66-67
+//                 levels; a small system's in one block, k_small_sums; a batch launches
+//                 kb_level_sums per level), children in the order of
+//                 TreeInitShader.comp:78-80; centre of mass as TreeMoveShader.comp:66-67
 //   quadrupole mode (accurate mode, moments.cuh): exact integer sums instead --
 //   k_mom_tiles   the sums of every tile of 1024 sorted slots
 //   k_mom_scan    their exclusive prefix at every slot
@@ -1165,6 +1166,107 @@ k_coop_sums(const uint32_t* __restrict__ level_count, const uint32_t* __restrict
     if (blockIdx.x == 0) top_sums_body(level_count, levels, n_al, skey, D, rec, kids, nodeinfo, msum, safe, bbox_mode, bpp);
 }
 
+// Monopole moments of a small system in one block: the records and child links go to shared
+// memory (a tree of more records is summed in global memory), and the levels, in the lists
+// that k_nodes left, follow one another with block barriers and shared-memory latency.  Every
+// node is computed exactly as by the per-level launches.  N = 3000: 17 us, against 33 in the
+// cooperative launch, most of it in its grid barriers; at 10,000, where the records no longer
+// fit, the launch takes 35.  (Larger systems as runs of slots a block, the nodes
+// across their boundaries summed by the last block, took 60 to 85 us at N = 500,000 against
+// 45: one SM's requests to L2 set the pace of the boundary nodes.)
+constexpr uint32_t kSmallRecords = 5632;     // 40 bytes each: 220 KB
+constexpr uint64_t kSmallSumsMax = 3072;     // particles
+constexpr uint32_t kSmallThreads = 1024;
+struct SmallSmem {
+    float4 rec[kSmallRecords];
+    uint4 kid[kSmallRecords];
+    float2 sum[kSmallRecords];   // mass moments of a summed node
+};
+
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_sums(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ level_count,
+             const uint32_t* __restrict__ levels, uint32_t n_al, const uint32_t* __restrict__ skey, int D, float4* rec,
+             const uint4* __restrict__ kids, const uint2* __restrict__ nodeinfo, float2* msum, int safe, int bbox_mode,
+             const BHParams* __restrict__ bpp, uint32_t cap) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    SmallSmem& g = *reinterpret_cast<SmallSmem*>(s_raw);
+    pdl_enter();
+    const BHParams bp = *bpp;
+    const uint32_t T = min(counts[0] + counts[1], cap);
+    if (!T) return;
+    if (T > kSmallRecords) {
+        for (int d = D; d >= 0; --d) {
+            const uint32_t cnt = min(level_count[d], level_cap(d, n_al));
+            const uint32_t* list = levels + level_off(d, n_al);
+            for (uint32_t t = threadIdx.x; t < cnt; t += kSmallThreads)
+                compute_node(list[t], D, safe, bbox_mode, bp, skey, rec, kids, nodeinfo, msum);
+            __syncthreads();
+        }
+        return;
+    }
+    for (uint32_t i = threadIdx.x; i < T; i += kSmallThreads) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&g.rec[i])),
+                     "l"(rec + i)
+                     : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&g.kid[i])),
+                     "l"(kids + i)
+                     : "memory");
+    }
+    uint32_t cnt = min(level_count[D], level_cap(D, n_al));
+    uint32_t at = threadIdx.x < cnt ? levels[level_off(D, n_al) + threadIdx.x] : 0u;  // the level's first node of this thread
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    for (int d = D; d >= 0; --d) {
+        const uint32_t here = cnt, mine = at;
+        if (d > 0) {  // the next level's, in flight meanwhile
+            cnt = min(level_count[d - 1], level_cap(d - 1, n_al));
+            at = threadIdx.x < cnt ? levels[level_off(d - 1, n_al) + threadIdx.x] : 0u;
+        }
+        for (uint32_t t = threadIdx.x; t < here; t += kSmallThreads) {
+            const uint32_t i = min(t == threadIdx.x ? mine : levels[level_off(d, n_al) + t], T - 1);
+            const uint4 kd = g.kid[i];
+            float sx = 0.0f, sy = 0.0f, sm = 0.0f;
+            const auto add = [&](float m, float mx, float my) {
+                sx = __fadd_rn(sx, mx);
+                sy = __fadd_rn(sy, my);
+                sm = __fadd_rn(sm, m);
+            };
+            if (kd.x == kKidFinest) {
+                const uint32_t leaves = kd.y < T ? min(kd.z, T - kd.y) : 0u;
+                for (uint32_t u = 0; u < leaves; ++u) {
+                    const float4 r = g.rec[kd.y + u];
+                    add(r.z, __fmul_rn(r.x, r.z), __fmul_rn(r.y, r.z));
+                }
+            } else {
+                const uint32_t kk[4] = {kd.x, kd.y, kd.z, kd.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (kk[u] == kKidNone) continue;
+                    const uint32_t c = min(kk[u] & ~kKidLeaf, T - 1);
+                    const float4 r = g.rec[c];
+                    if (kk[u] & kKidLeaf) {
+                        add(r.z, __fmul_rn(r.x, r.z), __fmul_rn(r.y, r.z));
+                    } else {
+                        const float2 m2 = g.sum[c];
+                        add(r.z, m2.x, m2.y);
+                    }
+                }
+            }
+            float cx = sx, cy = sy;
+            if (sm != 0.0f) {
+                cx = __fdiv_rn(sx, sm);
+                cy = __fdiv_rn(sy, sm);
+            }
+            const float rad = safe ? cell_bmax2(bbox_mode, bp, D, d, nodeinfo[i].x, cx, cy) : g.rec[i].w;
+            const float4 q = make_float4(cx, cy, sm, rad);
+            g.rec[i] = q;
+            g.sum[i] = make_float2(sx, sy);
+            rec[i] = q;
+        }
+        __syncthreads();  // level d is complete before level d - 1
+    }
+}
+
 __global__ void k_set_params(BHParams* __restrict__ out, BHParams v) { *out = v; }
 
 }  // namespace
@@ -1384,12 +1486,22 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     if (!w.quad) {  // monopole moments, level by level (the quadrupole mode has them from k_nodes)
         const int safe = (s->p.flags & GS_FLAG_SAFE_RADIUS) ? 1 : 0;
         const int bb = bbox ? 1 : 0;
-        const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm
-                                                                                : w.sums_per_sm;
-        GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, w.sms * per_sm, kCoopSumsThreads, st,
-                                  (const uint32_t*)(ctr + kCtrLevel), (const uint32_t*)w.levels, n, skey, w.depth,
-                                  w.rec, (const uint4*)w.kids, (const uint2*)w.nodeinfo, w.msum, safe, bb,
-                                  (const BHParams*)w.params, ctr + kCtrBarrier, s->d_err));
+        if (n <= kSmallSumsMax) {
+            GS_TRY_LAUNCH(cudaFuncSetAttribute(k_small_sums, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(SmallSmem)));
+            GS_TRY_LAUNCH(launch_shared(next_pdl(), k_small_sums, 1, kSmallThreads, (unsigned)sizeof(SmallSmem), st,
+                                        (const uint32_t*)(ctr + kCtrValid), (const uint32_t*)(ctr + kCtrLevel),
+                                        (const uint32_t*)w.levels, n, skey, w.depth, w.rec, (const uint4*)w.kids,
+                                        (const uint2*)w.nodeinfo, w.msum, safe, bb, (const BHParams*)w.params,
+                                        (uint32_t)w.cap));
+        } else {
+            const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm
+                                                                                    : w.sums_per_sm;
+            GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, w.sms * per_sm, kCoopSumsThreads, st,
+                                      (const uint32_t*)(ctr + kCtrLevel), (const uint32_t*)w.levels, n, skey, w.depth,
+                                      w.rec, (const uint4*)w.kids, (const uint2*)w.nodeinfo, w.msum, safe, bb,
+                                      (const BHParams*)w.params, ctr + kCtrBarrier, s->d_err));
+        }
         count_launch(s);
     }
     stage_end(s, kStageSums, profile);
