@@ -23,15 +23,16 @@
 //   monopole mode (the reference's rule):
 //   k_coop_sums   mass and mass-moment sums level by level, finest first (one cooperative
 //                 launch, a grid barrier between deep levels, one block for the top
-//                 levels; a small system's in one block, k_small_sums; a batch launches
-//                 kb_level_sums per level), children in the order of
-//                 TreeInitShader.comp:78-80; centre of mass as TreeMoveShader.comp:66-67
+//                 levels; a batch launches kb_level_sums per level), children in the order
+//                 of TreeInitShader.comp:78-80; centre of mass as TreeMoveShader.comp:66-67
 //   quadrupole mode (accurate mode, moments.cuh): exact integer sums instead --
 //   k_mom_tiles   the sums of every tile of 1024 sorted slots
 //   k_mom_scan    their exclusive prefix at every slot
 //   k_mom_nodes   each internal node's centre, mass, opening radius and second moments
 //                 from the prefix at its first slot and one past its last (k_nodes keeps
 //                 the end)
+//   k_small_tree  all of the above up to here for a small system alone, in one block (the
+//                 moments in monopole mode)
 //   k_force       ForceShader.comp:78-152 semantics: one warp walks the preorder records
 //                 for 32 consecutive sorted slots; a record is accepted only if every
 //                 lane satisfies radius <= d2 * theta^2; 32-record window staged in shared
@@ -229,6 +230,29 @@ inline int keygen_blocks(uint64_t n) {
     return (int)(b < 1 ? 1 : b > (uint64_t)kKeyBlocks ? kKeyBlocks : b);
 }
 
+// The key of particle i at q; one outside the fixed box is removed (InitShader.comp:110-117).
+// Counts it in `valid` and its mass m in `mbits`, the bits of the largest.
+__device__ __forceinline__ uint32_t particle_key(uint32_t i, float2 q, float m, int bbox_mode, const BHParams& p,
+                                                 float2* __restrict__ pos_in, float* mass_in,
+                                                 float2* __restrict__ pos_out, float* mass_out, uint32_t& valid,
+                                                 uint32_t& mbits) {
+    uint32_t key;
+    if (bbox_mode) {
+        key = spread_bits(bbox_cell(q.x, p.cx, p.scale, p.bits)) |
+              (spread_bits(bbox_cell(q.y, p.cy, p.scale, p.bits)) << 1);
+    } else if (!fixed_key(q.x, q.y, key)) {
+        const float2 gone = make_float2(-kSimSize * 2.0f, -kSimSize * 2.0f);
+        pos_in[i] = gone;
+        pos_out[i] = gone;
+        mass_in[i] = 0.0f;
+        mass_out[i] = 0.0f;
+        return kKeyRemovedSort;
+    }
+    ++valid;
+    if (m > 0.0f) mbits = max(mbits, __float_as_uint(m));
+    return key;
+}
+
 // mmax (quadrupole mode, else null): the largest mass after the removal, as float bits
 // (masses >= 0 order like their bits), for the grid of the exact moment sums.
 __device__ __forceinline__ void keygen_body(Blk blk, int bbox_mode, const BHParams* __restrict__ bp,
@@ -244,30 +268,8 @@ __device__ __forceinline__ void keygen_body(Blk blk, int bbox_mode, const BHPara
     if (bbox_mode) p = *bp;
     uint32_t valid = 0, mbits = 0;
     for (uint32_t i = blk.id * kKeyThreads + threadIdx.x; i < n; i += blk.count * kKeyThreads) {
-        float2 q = pos_in[i];
-        uint32_t key;
-        if (bbox_mode) {
-            key = spread_bits(bbox_cell(q.x, p.cx, p.scale, p.bits)) |
-                  (spread_bits(bbox_cell(q.y, p.cy, p.scale, p.bits)) << 1);
-            ++valid;
-            if (mmax) {
-                const float m = mass_in[i];
-                if (m > 0.0f) mbits = max(mbits, __float_as_uint(m));
-            }
-        } else if (fixed_key(q.x, q.y, key)) {
-            ++valid;
-            if (mmax) {
-                const float m = mass_in[i];
-                if (m > 0.0f) mbits = max(mbits, __float_as_uint(m));
-            }
-        } else {  // InitShader.comp:110-117
-            key = kKeyRemovedSort;
-            const float2 gone = make_float2(-kSimSize * 2.0f, -kSimSize * 2.0f);
-            pos_in[i] = gone;
-            pos_out[i] = gone;
-            mass_in[i] = 0.0f;
-            mass_out[i] = 0.0f;
-        }
+        const uint32_t key = particle_key(i, pos_in[i], mmax ? mass_in[i] : 0.0f, bbox_mode, p, pos_in, mass_in,
+                                          pos_out, mass_out, valid, mbits);
         keys[i] = key;
         for (int ps = 0; ps < passes; ++ps) atomicAdd(&sh[ps][(key >> (8 * ps)) & 255u], 1u);
     }
@@ -794,9 +796,30 @@ __device__ __forceinline__ uint32_t leaf_of(const uint32_t* skey, const uint32_t
     return t + E[t] + (uint32_t)(cmax >= cmin ? cmax - cmin + 1 : 0);
 }
 
-// One thread per sorted slot s: the particle leaf of s, and the slot of every internal
-// node that starts at s in the node -> slot map (internal ordinal j = E(s) + d - dmin(s),
-// record index s + j).
+// Sorted slot s: its particle leaf, and the slot of every internal node that starts at s in the
+// node -> slot map (internal ordinal j = E(s) + d - dmin(s), record index s + j).
+__device__ __forceinline__ void slot_records(uint32_t s, uint32_t i, const uint32_t* skey, const uint32_t* E,
+                                             uint32_t nv, int D, const float2* __restrict__ pos, const float* mass,
+                                             float4* __restrict__ rec, uint32_t* __restrict__ skip,
+                                             uint32_t* __restrict__ node_slot, uint64_t cap, uint32_t n_al,
+                                             int* __restrict__ err, const MomIn& mi, const MomScale& sc) {
+    const int dmin = slot_dmin(skey, s, D), dmax = slot_dmax(skey, s, nv, D);
+    const uint32_t Es = E[s];
+    const int e = dmax >= dmin ? dmax - dmin + 1 : 0;
+    const uint64_t leaf = (uint64_t)s + Es + e;
+    if (leaf >= cap || i >= n_al) {  // i >= n_al: only after a failed sort (error flag already set)
+        atomicOr(err, kErrTree);
+        return;
+    }
+    const float2 p = pos[i];
+    const float m = mass[i];
+    rec[leaf] = make_float4(p.x, p.y, m, 0.0f);
+    skip[leaf] = 1u;
+    if (mi.prefix) mi.qv[s] = mom_quantize(p, m, sc);
+    for (int k = 0; k < e; ++k) node_slot[Es + k] = s;
+}
+
+// One thread per sorted slot.
 __device__ __forceinline__ void records_body(Blk blk, const uint32_t* __restrict__ skey,
                                              const uint32_t* __restrict__ sidx, const uint32_t* __restrict__ E,
                                              const uint32_t* __restrict__ valid_count, int D,
@@ -807,27 +830,8 @@ __device__ __forceinline__ void records_body(Blk blk, const uint32_t* __restrict
     const uint32_t nv = *valid_count;
     MomScale sc;
     if (mi.prefix) sc = mom_scale(mi.bbox, *mi.bp, *mi.mmax);
-    for (uint32_t s = blk.id * 256 + threadIdx.x; s < nv; s += blk.count * 256) {
-        const int dmin = slot_dmin(skey, s, D), dmax = slot_dmax(skey, s, nv, D);
-        const uint32_t Es = E[s];
-        const int e = dmax >= dmin ? dmax - dmin + 1 : 0;
-        const uint64_t leaf = (uint64_t)s + Es + e;
-        if (leaf >= cap) {
-            atomicOr(err, kErrTree);
-            continue;
-        }
-        const uint32_t i = sidx[s];
-        if (i >= n_al) {  // only after a failed sort (error flag already set)
-            atomicOr(err, kErrTree);
-            continue;
-        }
-        const float2 p = pos[i];
-        const float m = mass[i];
-        rec[leaf] = make_float4(p.x, p.y, m, 0.0f);
-        skip[leaf] = 1u;
-        if (mi.prefix) mi.qv[s] = mom_quantize(p, m, sc);
-        for (int k = 0; k < e; ++k) node_slot[Es + k] = s;
-    }
+    for (uint32_t s = blk.id * 256 + threadIdx.x; s < nv; s += blk.count * 256)
+        slot_records(s, sidx[s], skey, E, nv, D, pos, mass, rec, skip, node_slot, cap, n_al, err, mi, sc);
 }
 
 // The costly groups of the step (relative criterion, quadrupole mode): a flag per group
@@ -900,19 +904,76 @@ __host__ __device__ __forceinline__ uint32_t level_off(int d, uint32_t n_al) {
     return o;
 }
 
-// One thread per internal node (d, s): skip (the reference's count.y), the level radius
-// of TreeMoveShader.comp:70-71, the child descriptors, and the node's entry in the list
-// of its level (slots reserved per block: a shared histogram, one atomic per level).
-// Quadrupole mode (mi.prefix set): the record itself is left to k_mom_nodes, which reads
-// the node's end slot from mi.nend.
+// Internal node j, which starts at slot s: skip (the reference's count.y), the level radius of
+// TreeMoveShader.comp:70-71 and the child descriptors; returns its level, or -1 on a failed tree.
+// Quadrupole mode (mi.prefix set): the record itself is left to k_mom_nodes, which reads the
+// node's end slot from mi.nend.
+__device__ __forceinline__ int layout_node(uint32_t j, uint32_t s, const uint32_t* skey, const uint32_t* E, uint32_t nv,
+                                           int D, float radius0, float4* __restrict__ rec, uint32_t* __restrict__ skip,
+                                           uint4* __restrict__ kids, uint2* __restrict__ nodeinfo, uint64_t cap,
+                                           int* __restrict__ err, const MomIn& mi) {
+    const uint32_t at = s + j;
+    if (s >= nv || at >= cap) {  // only after a failed sort or scan (error flag already set)
+        atomicOr(err, kErrTree);
+        return -1;
+    }
+    const int d = slot_dmin(skey, s, D) + (int)(j - E[s]);
+    const int shift = 2 * (D - d);
+    const uint32_t ks = skey[s];
+    uint32_t end;
+    if (d == D) {
+        end = cell_end(skey, s + 1, nv, shift, ks >> shift);
+        kids[at] = make_uint4(kKidFinest, at + 1, end - s, 0u);  // all children are leaves
+    } else {
+        // The cell ends where its level-d prefix changes (galloping search); its
+        // level-(d+1) cells, in Morton order, are the runs of prefix 4p + c,
+        // c = 0..3, inside it.  The ends of the first three are found by three
+        // binary searches run in lockstep (their loads overlap), so a large cell
+        // costs about three times log2(size) dependent loads, not four gallops.
+        end = cell_end(skey, s + 1, nv, shift, ks >> shift);
+        const int cshift = 2 * (D - d - 1);
+        const uint32_t p4 = (ks >> shift) << 2;
+        uint32_t lo[3] = {s, s, s}, hi[3] = {end, end, end};
+        while (lo[0] < hi[0] || lo[1] < hi[1] || lo[2] < hi[2]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (lo[c] < hi[c]) {
+                    const uint32_t mid = lo[c] + ((hi[c] - lo[c]) >> 1);
+                    if ((skey[mid] >> cshift) <= p4 + (uint32_t)c) lo[c] = mid + 1;
+                    else hi[c] = mid;
+                }
+            }
+        }
+        const uint32_t cend[4] = {lo[0], lo[1], lo[2], end};
+        uint32_t kid[4] = {kKidNone, kKidNone, kKidNone, kKidNone};
+        uint32_t nk = 0, t = s;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t tend = cend[c];
+            if (tend == t) continue;  // no particle in this child cell
+            if (tend - t >= 2) kid[nk] = t + E[t] + (uint32_t)(d + 1 - slot_dmin(skey, t, D));  // node (d+1, t)
+            else kid[nk] = leaf_of(skey, E, t, nv, D) | kKidLeaf;
+            ++nk;
+            t = tend;
+        }
+        kids[at] = make_uint4(kid[0], kid[1], kid[2], kid[3]);
+    }
+    if (mi.prefix) mi.nend[j] = end;
+    else rec[at] = make_float4(0.0f, 0.0f, 0.0f, __fdiv_rn(radius0, (float)(1u << (2 * d))));
+    skip[at] = end + E[end] - at;
+    nodeinfo[at] = make_uint2(ks, (uint32_t)d);  // a key of the cell, its level
+    return d;
+}
+
+// One thread per internal node: its layout, and its entry in the list of its level (slots
+// reserved per block: a shared histogram, one atomic per level).
 __device__ __forceinline__ void nodes_body(Blk blk, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ E,
                                            const uint32_t* __restrict__ counts, int D,
                                            const BHParams* __restrict__ bp, const uint32_t* __restrict__ node_slot,
                                            float4* __restrict__ rec, uint32_t* __restrict__ skip,
                                            uint4* __restrict__ kids, uint2* __restrict__ nodeinfo,
                                            uint32_t* __restrict__ level_count, uint32_t* __restrict__ levels,
-                                           uint32_t n_al, uint64_t cap, int* __restrict__ err, const MomIn& mi,
-                                           float4* __restrict__ quad, int safe) {
+                                           uint32_t n_al, uint64_t cap, int* __restrict__ err, const MomIn& mi) {
     __shared__ uint32_t s_cnt[16], s_base[16];
     const uint32_t nv = counts[0], M = counts[1];
     const float radius0 = bp->radius0;
@@ -928,56 +989,8 @@ __device__ __forceinline__ void nodes_body(Blk blk, const uint32_t* __restrict__
         if (j < M) {
             const uint32_t s = node_slot[j];
             at = s + j;
-            if (s >= nv || at >= cap) {  // only after a failed sort or scan (error flag already set)
-                atomicOr(err, kErrTree);
-            } else {
-                d = slot_dmin(skey, s, D) + (int)(j - E[s]);
-                const int shift = 2 * (D - d);
-                const uint32_t ks = skey[s];
-                uint32_t end;
-                if (d == D) {
-                    end = cell_end(skey, s + 1, nv, shift, ks >> shift);
-                    kids[at] = make_uint4(kKidFinest, at + 1, end - s, 0u);  // all children are leaves
-                } else {
-                    // The cell ends where its level-d prefix changes (galloping search); its
-                    // level-(d+1) cells, in Morton order, are the runs of prefix 4p + c,
-                    // c = 0..3, inside it.  The ends of the first three are found by three
-                    // binary searches run in lockstep (their loads overlap), so a large cell
-                    // costs about three times log2(size) dependent loads, not four gallops.
-                    end = cell_end(skey, s + 1, nv, shift, ks >> shift);
-                    const int cshift = 2 * (D - d - 1);
-                    const uint32_t p4 = (ks >> shift) << 2;
-                    uint32_t lo[3] = {s, s, s}, hi[3] = {end, end, end};
-                    while (lo[0] < hi[0] || lo[1] < hi[1] || lo[2] < hi[2]) {
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            if (lo[c] < hi[c]) {
-                                const uint32_t mid = lo[c] + ((hi[c] - lo[c]) >> 1);
-                                if ((skey[mid] >> cshift) <= p4 + (uint32_t)c) lo[c] = mid + 1;
-                                else hi[c] = mid;
-                            }
-                        }
-                    }
-                    const uint32_t cend[4] = {lo[0], lo[1], lo[2], end};
-                    uint32_t kid[4] = {kKidNone, kKidNone, kKidNone, kKidNone};
-                    uint32_t nk = 0, t = s;
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint32_t tend = cend[c];
-                        if (tend == t) continue;  // no particle in this child cell
-                        if (tend - t >= 2) kid[nk] = t + E[t] + (uint32_t)(d + 1 - slot_dmin(skey, t, D));  // node (d+1, t)
-                        else kid[nk] = leaf_of(skey, E, t, nv, D) | kKidLeaf;
-                        ++nk;
-                        t = tend;
-                    }
-                    kids[at] = make_uint4(kid[0], kid[1], kid[2], kid[3]);
-                }
-                if (mi.prefix) mi.nend[j] = end;
-                else rec[at] = make_float4(0.0f, 0.0f, 0.0f, __fdiv_rn(radius0, (float)(1u << (2 * d))));
-                skip[at] = end + E[end] - at;
-                nodeinfo[at] = make_uint2(ks, (uint32_t)d);  // a key of the cell, its level
-                if (lists) rank = atomicAdd(&s_cnt[d], 1u);
-            }
+            d = layout_node(j, s, skey, E, nv, D, radius0, rec, skip, kids, nodeinfo, cap, err, mi);
+            if (lists && d >= 0) rank = atomicAdd(&s_cnt[d], 1u);
         }
         if (!lists) continue;
         __syncthreads();
@@ -1032,10 +1045,10 @@ k_nodes(const uint32_t* __restrict__ skey, const uint32_t* __restrict__ E, const
         int D, const BHParams* __restrict__ bp, const uint32_t* __restrict__ node_slot, float4* __restrict__ rec,
         uint32_t* __restrict__ skip, uint4* __restrict__ kids, uint2* __restrict__ nodeinfo,
         uint32_t* __restrict__ level_count, uint32_t* __restrict__ levels, uint32_t n_al, uint64_t cap,
-        int* __restrict__ err, MomIn mi, float4* __restrict__ quad, int safe) {
+        int* __restrict__ err, MomIn mi) {
     pdl_enter();
     nodes_body(grid_blk(), skey, E, counts, D, bp, node_slot, rec, skip, kids, nodeinfo, level_count, levels, n_al,
-               cap, err, mi, quad, safe);
+               cap, err, mi);
 }
 
 // One child's contribution: mass, centre of mass and mass moments.  Loads go through L2
@@ -1166,104 +1179,433 @@ k_coop_sums(const uint32_t* __restrict__ level_count, const uint32_t* __restrict
     if (blockIdx.x == 0) top_sums_body(level_count, levels, n_al, skey, D, rec, kids, nodeinfo, msum, safe, bbox_mode, bpp);
 }
 
-// Monopole moments of a small system in one block: the records and child links go to shared
-// memory (a tree of more records is summed in global memory), and the levels, in the lists
-// that k_nodes left, follow one another with block barriers and shared-memory latency.  Every
-// node is computed exactly as by the per-level launches.  N = 3000: 17 us, against 33 in the
-// cooperative launch, most of it in its grid barriers; at 10,000, where the records no longer
-// fit, the launch takes 35.  (Larger systems as runs of slots a block, the nodes
-// across their boundaries summed by the last block, took 60 to 85 us at N = 500,000 against
-// 45: one SM's requests to L2 set the pace of the boundary nodes.)
-constexpr uint32_t kSmallRecords = 5632;     // 40 bytes each: 220 KB
-constexpr uint64_t kSmallSumsMax = 3072;     // particles
-constexpr uint32_t kSmallThreads = 1024;
-struct SmallSmem {
-    float4 rec[kSmallRecords];
-    uint4 kid[kSmallRecords];
-    float2 sum[kSmallRecords];   // mass moments of a summed node
+// ------------------------------------------------------------------------------------
+// small systems: keys, sort, scan, records, node layout and monopole moments in one block
+// ------------------------------------------------------------------------------------
+// For a small system each of those stages is a few thousand operations behind a launch, a
+// histogram through global memory, a look-back, chains of dependent L2 loads or a grid barrier.
+// One block does them all in shared memory: KPT particles a thread, ranks from ballots, the ends
+// of the nodes by binary search over the block's keys, every child from those ends without a
+// search, the moments level by level with block barriers.  The tree is the separate stages' bit
+// for bit.  Bound by the one SM's issue (ballots) and its scattered record stores.  A step of
+// the reference rule against the separate stages: 1,000 particles 38.8 and 55.9 us, 3,000 50.3
+// and 69.0, 6,000 64.9 and 88.5, 8,000 102 and 119; with quadrupole moments, which the separate
+// kernels go on to sum, 1,000 58.2 and 63.9, 3,000 80.1 and 83.8, 4,090 87.9 and 87.8, 8,000 103
+// and 85.
+constexpr uint32_t kTreeThreads = 1024, kTreeWarps = kTreeThreads / 32;
+constexpr uint64_t kTreeSmallMax = 8192;      // particles: eight a thread
+constexpr uint64_t kTreeSmallQuadMax = 3072;  // in quadrupole mode
+
+template <int KPT>
+struct TreeSmem {
+    static constexpr uint32_t kN = kTreeThreads * KPT;
+    float2 pos[kN];  // by particle; for the moments by slot: mass moments and masses of the
+    float mass[kN];  // slot's leaf, then of the coarsest node summed so far that starts there
+    uint32_t key[kN];  // by sorted slot
+    uint16_t val[kN];  // ... its particle; then the nodes by level
+    union {
+        uint32_t hist[kTreeWarps][256];  // sort: a warp's count, then first place, of each digit
+        struct {
+            uint32_t E[kN + 4];              // exclusive scan of the nodes that start at a slot
+            uint16_t nslot[kN], nend[kN];  // an internal node's first slot and one past its last
+        };
+    };
+    uint32_t part[4][256];  // sort: the counts of eight warps
+    uint32_t start[256];
+    uint32_t warp[kTreeWarps];
+    uint32_t level[16], level_first[16];  // nodes of a level, and where its list starts
+    uint32_t valid, mbits;
+    BHParams box;
 };
 
-__global__ void __launch_bounds__(kSmallThreads)
-k_small_sums(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ level_count,
-             const uint32_t* __restrict__ levels, uint32_t n_al, const uint32_t* __restrict__ skey, int D, float4* rec,
-             const uint4* __restrict__ kids, const uint2* __restrict__ nodeinfo, float2* msum, int safe, int bbox_mode,
-             const BHParams* __restrict__ bpp, uint32_t cap) {
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    SmallSmem& g = *reinterpret_cast<SmallSmem*>(s_raw);
-    pdl_enter();
-    const BHParams bp = *bpp;
-    const uint32_t T = min(counts[0] + counts[1], cap);
-    if (!T) return;
-    if (T > kSmallRecords) {
-        for (int d = D; d >= 0; --d) {
-            const uint32_t cnt = min(level_count[d], level_cap(d, n_al));
-            const uint32_t* list = levels + level_off(d, n_al);
-            for (uint32_t t = threadIdx.x; t < cnt; t += kSmallThreads)
-                compute_node(list[t], D, safe, bbox_mode, bp, skey, rec, kids, nodeinfo, msum);
-            __syncthreads();
-        }
-        return;
+struct SmallTree {
+    float2* pos_in;
+    float* mass_in;
+    float2* pos_out;
+    float* mass_out;
+    uint32_t n;
+    int bbox, passes, D, safe;
+    int links;  // the traversal or k_mom_nodes reads the child descriptors
+    uint32_t* counters;
+    BHParams* params;
+    const uint32_t* ext_in;  // bounding box: the extents of the input and the output set
+    uint32_t* ext_out;
+    uint32_t *keys, *idx;
+    float4* rec;
+    uint32_t* skip;
+    uint4* kids;
+    uint2* nodeinfo;
+    uint32_t *node_slot, *levels;
+    float2* msum;
+    uint64_t cap;
+    int* err;
+    MomIn mi;
+};
+
+// The lanes of the warp whose low BITS bits of d equal this lane's.  A ballot per bit, and they
+// overlap over a thread's keys: match_any takes a turn for every distinct digit (3,000 keys:
+// three passes in 18.3 thousand cycles, with match_any 20.5 to 26.7).
+template <int BITS>
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d) {
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < BITS; ++b) {
+        uint32_t same;  // the lanes whose bit b equals this lane's
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x;\n\tand.b32 x, %1, %2;\n\tsetp.ne.u32 p, x, 0;\n\t"
+                     "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
+                     : "=r"(same)
+                     : "r"(d), "r"(1u << b));
+        peers &= same;
     }
-    for (uint32_t i = threadIdx.x; i < T; i += kSmallThreads) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&g.rec[i])),
-                     "l"(rec + i)
-                     : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&g.kid[i])),
-                     "l"(kids + i)
-                     : "memory");
+    return peers;
+}
+
+// One stable pass over the block's keys by the BITS-bit digit at `shift`: a thread's keys are
+// those at warp * 32 KPT + 32 j + lane.
+template <int BITS, int KPT>
+__device__ __forceinline__ void tree_sort_pass(TreeSmem<KPT>& g, uint32_t (&key)[KPT], uint32_t (&val)[KPT], int shift) {
+    constexpr uint32_t kMask = (1u << BITS) - 1u;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    uint4* clear = reinterpret_cast<uint4*>(&g.hist[warp][0]);
+    clear[lane] = clear[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t peers[KPT], rank[KPT];
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) peers[j] = digit_peers<BITS>(key[j] >> shift);
+    __syncwarp();
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        uint32_t& h = g.hist[warp][(key[j] >> shift) & kMask];
+        const uint32_t before = h;
+        rank[j] = before + __popc(peers[j] & lt);
+        __syncwarp();
+        if (!(peers[j] & lt)) h = before + __popc(peers[j]);
+        __syncwarp();
     }
-    uint32_t cnt = min(level_count[D], level_cap(D, n_al));
-    uint32_t at = threadIdx.x < cnt ? levels[level_off(D, n_al) + threadIdx.x] : 0u;  // the level's first node of this thread
-    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    for (int d = D; d >= 0; --d) {
-        const uint32_t here = cnt, mine = at;
-        if (d > 0) {  // the next level's, in flight meanwhile
-            cnt = min(level_count[d - 1], level_cap(d - 1, n_al));
-            at = threadIdx.x < cnt ? levels[level_off(d - 1, n_al) + threadIdx.x] : 0u;
+    const uint32_t q = t >> 8, d = t & 255u;  // thread: digit d of warps 8 q .. 8 q + 7
+    uint32_t first[8], sum = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        first[w] = sum;
+        sum += g.hist[8 * q + w][d];
+    }
+    g.part[q][d] = sum;
+    __syncthreads();
+    if (t < 256) {
+        const uint32_t tot = g.part[0][t] + g.part[1][t] + g.part[2][t] + g.part[3][t];
+        uint32_t x = tot;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)lane >= o) x += y;
         }
-        for (uint32_t t = threadIdx.x; t < here; t += kSmallThreads) {
-            const uint32_t i = min(t == threadIdx.x ? mine : levels[level_off(d, n_al) + t], T - 1);
-            const uint4 kd = g.kid[i];
-            float sx = 0.0f, sy = 0.0f, sm = 0.0f;
-            const auto add = [&](float m, float mx, float my) {
-                sx = __fadd_rn(sx, mx);
-                sy = __fadd_rn(sy, my);
-                sm = __fadd_rn(sm, m);
-            };
-            if (kd.x == kKidFinest) {
-                const uint32_t leaves = kd.y < T ? min(kd.z, T - kd.y) : 0u;
-                for (uint32_t u = 0; u < leaves; ++u) {
-                    const float4 r = g.rec[kd.y + u];
-                    add(r.z, __fmul_rn(r.x, r.z), __fmul_rn(r.y, r.z));
-                }
+        g.start[t] = x - tot;
+        if (lane == 31) g.warp[warp] = x;
+    }
+    __syncthreads();
+    uint32_t base = g.start[d];
+#pragma unroll
+    for (uint32_t w = 0; w < 7; ++w) base += w < d >> 5 ? g.warp[w] : 0u;
+#pragma unroll
+    for (uint32_t p = 0; p < 3; ++p) base += p < q ? g.part[p][d] : 0u;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) g.hist[8 * q + w][d] = base + first[w];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t to = g.hist[warp][(key[j] >> shift) & kMask] + rank[j];
+        g.key[to] = key[j];
+        g.val[to] = (uint16_t)val[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t i = (warp * KPT + j) * 32 + lane;
+        key[j] = g.key[i];
+        val[j] = g.val[i];
+    }
+}
+
+// This thread's node of level d (none: -1) among those of its level that the block has counted
+// so far: the level above its place there.  Every lane of the warp must call it.
+__device__ __forceinline__ uint32_t tree_place(uint32_t* level, int d) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    const int lead = __ffs(peers) - 1;
+    uint32_t first = 0;
+    if (d >= 0 && (int)lane == lead) first = atomicAdd(&level[d], (uint32_t)__popc(peers));
+    first = __shfl_sync(0xffffffffu, first, lead);
+    return (uint32_t)d << 16 | (first + __popc(peers & ((1u << lane) - 1u)));
+}
+
+// Node layout (and, in monopole mode, moments) of a tree with more nodes than the block's
+// shared memory holds, in global memory as the separate kernels do it.
+__device__ __noinline__ void tree_layout_general(const SmallTree& a, const uint32_t* key, const uint32_t* E,
+                                                 uint32_t* level, uint32_t nv, uint32_t M, const BHParams& box) {
+    const bool quad = a.mi.prefix != nullptr;
+    for (uint32_t j0 = 0; j0 < M; j0 += kTreeThreads) {
+        const uint32_t j = j0 + threadIdx.x;
+        int d = -1;
+        uint32_t s = 0;
+        if (j < M && j < a.cap) {
+            s = a.node_slot[j];
+            d = layout_node(j, s, key, E, nv, a.D, box.radius0, a.rec, a.skip, a.kids, a.nodeinfo, a.cap, a.err, a.mi);
+        }
+        if (quad) continue;
+        const uint32_t slot = tree_place(level, d) & 0xffffu;
+        if (d < 0) continue;
+        if (slot < level_cap(d, a.n)) a.levels[level_off(d, a.n) + slot] = s + j;
+        else atomicOr(a.err, kErrTree);
+    }
+    if (quad) return;
+    __syncthreads();
+    for (int d = a.D; d >= 0; --d) {
+        const uint32_t cnt = min(level[d], level_cap(d, a.n));
+        for (uint32_t i = threadIdx.x; i < cnt; i += kTreeThreads)
+            compute_node(a.levels[level_off(d, a.n) + i], a.D, a.safe, a.bbox, box, a.keys, a.rec, a.kids, a.nodeinfo,
+                         a.msum);
+        __syncthreads();
+    }
+}
+
+template <int KPT>
+__global__ void __launch_bounds__(kTreeThreads) k_small_tree(SmallTree a) {
+    static_assert(kTreeThreads * KPT < 65536, "16-bit slots");
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    TreeSmem<KPT>& g = *reinterpret_cast<TreeSmem<KPT>*>(s_raw);
+    constexpr uint32_t N = TreeSmem<KPT>::kN;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    pdl_enter();
+    if (t < kCtrCount) a.counters[t] = 0u;
+    if (t < 16) g.level[t] = 0u;
+    if (t == 0) {
+        g.valid = g.mbits = 0u;
+        if (a.bbox) {
+            g.box = bbox_params(ext_decode(a.ext_in), a.D);
+            *a.params = g.box;
+            for (int j = 0; j < 4; ++j) a.ext_out[j] = 0xFFFFFFFFu;
+        } else {
+            g.box = *a.params;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t i = (warp * KPT + j) * 32 + lane;
+        if (i < a.n) {
+            g.pos[i] = a.pos_in[i];
+            g.mass[i] = a.mass_in[i];
+        }
+    }
+    __syncthreads();
+    const BHParams box = g.box;
+    uint32_t key[KPT], val[KPT], valid = 0, mbits = 0;
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t i = val[j] = (warp * KPT + j) * 32 + lane;
+        // past the end: the last places of every pass
+        key[j] = i < a.n ? particle_key(i, g.pos[i], g.mass[i], a.bbox, box, a.pos_in, a.mass_in, a.pos_out,
+                                        a.mass_out, valid, mbits)
+                         : 0xffffffffu;
+    }
+    valid = __reduce_add_sync(0xffffffffu, valid);
+    mbits = __reduce_max_sync(0xffffffffu, mbits);
+    if (lane == 0) {
+        atomicAdd(&g.valid, valid);
+        atomicMax(&g.mbits, mbits);
+    }
+    if (a.bbox) {
+        for (int ps = 0; ps < a.passes; ++ps) tree_sort_pass<8>(g, key, val, 8 * ps);
+    } else {  // the 20 bits of a fixed-box key and the bit of removed particles
+        for (int ps = 0; ps < 3; ++ps) tree_sort_pass<7>(g, key, val, 7 * ps);
+    }
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t i = (warp * KPT + j) * 32 + lane;
+        if (i < a.n) {
+            a.keys[i] = key[j];
+            a.idx[i] = val[j];
+        }
+    }
+    // internal nodes that start at each slot, and their exclusive scan: KPT consecutive slots
+    const uint32_t nv = g.valid, s0 = t * KPT;
+    uint32_t k[KPT + 2], e[KPT], sum = 0;
+    k[0] = t ? g.key[s0 - 1] : 0u;
+    k[KPT + 1] = t + 1 < kTreeThreads ? g.key[s0 + KPT] : 0u;
+#pragma unroll
+    for (int j = 0; j < KPT; j += 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(&g.key[s0 + j]);
+        k[j + 1] = v.x;
+        k[j + 2] = v.y;
+    }
+#pragma unroll
+    for (int j = 0; j < KPT; ++j) {
+        const uint32_t s = s0 + j;
+        int c = 0;
+        if (s < nv) {
+            const int dmin = s == 0 ? 0 : common_bits(k[j], k[j + 1], 2 * a.D) / 2 + 1;
+            const int dmax = s + 1 < nv ? common_bits(k[j + 1], k[j + 2], 2 * a.D) / 2 : -1;
+            c = dmax - dmin + 1;
+        }
+        e[j] = sum;
+        sum += c > 0 ? (uint32_t)c : 0u;
+    }
+    uint32_t x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)lane >= o) x += y;
+    }
+    if (lane == 31) g.warp[warp] = x;
+    __syncthreads();
+    uint32_t w = g.warp[lane];  // every warp scans the warps' sums
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+        if ((int)lane >= o) w += y;
+    }
+    const uint32_t M = __shfl_sync(0xffffffffu, w, 31);  // internal nodes
+    const uint32_t before = (warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0u) + x - sum;
+#pragma unroll
+    for (int j = 0; j < KPT; j += 2)
+        *reinterpret_cast<uint2*>(&g.E[s0 + j]) = make_uint2(before + e[j], before + e[j + 1]);
+    if (t == 0) g.E[N] = M;
+    __syncthreads();
+    // particle leaves, and the slot of every node
+    const bool quad = a.mi.prefix != nullptr, fits = M <= N;  // the nodes' slots and ends fit the block
+    MomScale sc;
+    if (quad) sc = mom_scale(a.bbox, box, g.mbits);
+    float mx[KPT], my[KPT], mm[KPT];
+#pragma unroll
+    for (int r = 0; r < KPT; ++r) {
+        const uint32_t s = r * kTreeThreads + t;
+        mx[r] = my[r] = mm[r] = 0.0f;
+        if (s >= nv) continue;
+        const uint32_t e0 = g.E[s], e1 = g.E[s + 1], leaf = s + e1, i = g.val[s];
+        if (leaf >= a.cap) {
+            atomicOr(a.err, kErrTree);
+            continue;
+        }
+        const float2 p = g.pos[i];
+        const float m = g.mass[i];
+        mx[r] = __fmul_rn(p.x, m);
+        my[r] = __fmul_rn(p.y, m);
+        mm[r] = m;
+        a.rec[leaf] = make_float4(p.x, p.y, m, 0.0f);
+        a.skip[leaf] = 1u;
+        if (quad) a.mi.qv[s] = mom_quantize(p, m, sc);
+        for (uint32_t j = e0; j < e1; ++j) {
+            if (quad || !fits) a.node_slot[j] = s;
+            if (fits) g.nslot[j] = (uint16_t)s;
+        }
+    }
+    __syncthreads();
+    if (!fits) {
+        tree_layout_general(a, g.key, g.E, g.level, nv, M, box);
+    } else {
+        // one past the last slot of every node: a binary search over the block's keys
+        uint32_t top = 1, place[KPT];
+        while (2 * top < nv) top *= 2;
+#pragma unroll
+        for (int r = 0; r < KPT; ++r) {
+            const uint32_t j = r * kTreeThreads + t;
+            int d = -1;
+            if (j < M) {
+                uint32_t at = g.nslot[j];
+                d = slot_dmin(g.key, at, a.D) + (int)(j - g.E[at]);
+                const int shift = 2 * (a.D - d);
+                const uint32_t pre = g.key[at] >> shift;
+                for (uint32_t step = top; step; step >>= 1)
+                    if (at + step < nv && g.key[at + step] >> shift == pre) at += step;
+                g.nend[j] = (uint16_t)(at + 1);
+            }
+            if (!quad) place[r] = tree_place(g.level, d);
+        }
+        if (!quad) {  // by slot
+#pragma unroll
+            for (int r = 0; r < KPT; ++r) {
+                const uint32_t s = r * kTreeThreads + t;
+                g.pos[s] = make_float2(mx[r], my[r]);
+                g.mass[s] = mm[r];
+            }
+        }
+        __syncthreads();
+        if (t < 16) {
+            uint32_t first = 0;
+            for (uint32_t l = 0; l < t; ++l) first += g.level[l];
+            g.level_first[t] = first;
+        }
+        for (uint32_t j = t; j < M; j += kTreeThreads) {
+            const uint32_t s = g.nslot[j], end = g.nend[j], at = s + j;
+            const int d = slot_dmin(g.key, s, a.D) + (int)(j - g.E[s]);
+            if (at >= a.cap) {
+                atomicOr(a.err, kErrTree);
+                continue;
+            }
+            if (quad) a.mi.nend[j] = end;
+            a.skip[at] = end + g.E[end] - at;
+            if (!a.links) continue;
+            a.nodeinfo[at] = make_uint2(g.key[s], (uint32_t)d);  // a key of the cell, its level
+            if (d == a.D) {
+                a.kids[at] = make_uint4(kKidFinest, at + 1, end - s, 0u);  // all children are leaves
             } else {
-                const uint32_t kk[4] = {kd.x, kd.y, kd.z, kd.w};
+                // the children follow one another: a child at slot c is a node if one of its level
+                // starts there (the next at the node's own slot, the first at another) and ends
+                // where that ends, or else is the slot's leaf
+                uint32_t kid[4] = {kKidNone, kKidNone, kKidNone, kKidNone}, c = s, o = j + 1;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    if (kk[u] == kKidNone) continue;
-                    const uint32_t c = min(kk[u] & ~kKidLeaf, T - 1);
-                    const float4 r = g.rec[c];
-                    if (kk[u] & kKidLeaf) {
-                        add(r.z, __fmul_rn(r.x, r.z), __fmul_rn(r.y, r.z));
-                    } else {
-                        const float2 m2 = g.sum[c];
-                        add(r.z, m2.x, m2.y);
-                    }
+                    if (c >= end) continue;
+                    const uint32_t e1 = g.E[c + 1];
+                    kid[u] = o < e1 ? c + o : (c + e1) | kKidLeaf;
+                    c = o < e1 ? g.nend[o] : c + 1;
+                    o = g.E[c];
                 }
+                a.kids[at] = make_uint4(kid[0], kid[1], kid[2], kid[3]);
             }
-            float cx = sx, cy = sy;
-            if (sm != 0.0f) {
-                cx = __fdiv_rn(sx, sm);
-                cy = __fdiv_rn(sy, sm);
-            }
-            const float rad = safe ? cell_bmax2(bbox_mode, bp, D, d, nodeinfo[i].x, cx, cy) : g.rec[i].w;
-            const float4 q = make_float4(cx, cy, sm, rad);
-            g.rec[i] = q;
-            g.sum[i] = make_float2(sx, sy);
-            rec[i] = q;
         }
-        __syncthreads();  // level d is complete before level d - 1
+        if (!quad) {
+            __syncthreads();  // level_first
+#pragma unroll
+            for (int r = 0; r < KPT; ++r) {
+                const uint32_t j = r * kTreeThreads + t;
+                if (j < M) g.val[g.level_first[place[r] >> 16] + (place[r] & 0xffffu)] = (uint16_t)j;
+            }
+            __syncthreads();
+            // Mass, mass moments and centre of every node, finest level first, children in Morton
+            // order (compute_node's sums).  A node's moments take the place of its first child's,
+            // which nothing else reads.
+            for (int d = a.D; d >= 0; --d) {
+                const uint32_t cnt = g.level[d], first = g.level_first[d];
+                for (uint32_t i = t; i < cnt; i += kTreeThreads) {
+                    const uint32_t j = g.val[first + i], s = g.nslot[j], end = g.nend[j], at = s + j;
+                    float sx = 0.0f, sy = 0.0f, sm = 0.0f;
+                    for (uint32_t c = s, o = j + 1; c < end; o = g.E[c]) {
+                        const float2 q = g.pos[c];
+                        sx = __fadd_rn(sx, q.x);
+                        sy = __fadd_rn(sy, q.y);
+                        sm = __fadd_rn(sm, g.mass[c]);
+                        c = o < g.E[c + 1] ? g.nend[o] : c + 1;
+                    }
+                    g.pos[s] = make_float2(sx, sy);
+                    g.mass[s] = sm;
+                    float cx = sx, cy = sy;
+                    if (sm != 0.0f) {
+                        cx = __fdiv_rn(sx, sm);
+                        cy = __fdiv_rn(sy, sm);
+                    }
+                    const float rad = a.safe ? cell_bmax2(a.bbox, box, a.D, d, g.key[s], cx, cy)
+                                             : __fdiv_rn(box.radius0, (float)(1u << (2 * d)));
+                    if (at < a.cap) a.rec[at] = make_float4(cx, cy, sm, rad);
+                }
+                __syncthreads();  // level d is complete before level d - 1
+            }
+        }
+    }
+    __syncthreads();
+    if (t < 16) a.counters[kCtrLevel + t] = g.level[t];
+    if (t == 0) {
+        a.counters[kCtrValid] = nv;
+        a.counters[kCtrInternal] = M;
+        a.counters[kCtrMaxMass] = g.mbits;
     }
 }
 
@@ -1381,9 +1723,9 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     cudaStream_t st = s->stream;
     const uint32_t n = (uint32_t)s->n_al;
     const bool bbox = s->p.box_mode == GS_BOX_BOUNDING;
-    cudaError_t e = cudaMemsetAsync(w.zero_base, 0, w.zero_bytes, st);
-    if (e != cudaSuccess) return e;
     uint32_t* ctr = w.counters;
+    // one block from the keys to the node layout and the monopole moments
+    const bool small = n <= (w.quad ? kTreeSmallQuadMax : kTreeSmallMax);
     // programmatic launches everywhere except right after the memset, and not while
     // stage events sit between the launches
     const bool pdl = !profile;
@@ -1393,41 +1735,9 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
         first = false;
         return r;
     };
-    stage_begin(s, kStageKeys, profile);
-    if (bbox) {  // the box from the extent carried with the input set
-        GS_TRY_LAUNCH(launch(next_pdl(), k_ext_keys, keygen_blocks(n), kKeyThreads, st, s->pos[in], s->mass[in],
-                             s->pos[out], s->mass[out], n, w.keys[0], w.hist, w.passes, ctr + kCtrValid, w.params,
-                             (const uint32_t*)(w.ext + 4 * in), w.ext + 4 * out, w.depth,
-                             w.quad ? ctr + kCtrMaxMass : nullptr));
-    } else {
-        GS_TRY_LAUNCH(launch(next_pdl(), k_keygen, keygen_blocks(n), kKeyThreads, st, 0,
-                             (const BHParams*)w.params, s->pos[in], s->mass[in], s->pos[out], s->mass[out], n,
-                             w.keys[0], w.hist, w.passes, ctr + kCtrValid, w.quad ? ctr + kCtrMaxMass : nullptr));
-    }
-    count_launch(s);
-    stage_end(s, kStageKeys, profile);
-    stage_begin(s, kStageSort, profile);
-    const uint32_t kpt = sort_kpt(n, s->shape);
-    for (int ps = 0; ps < w.passes; ++ps) {
-        const int a = ps & 1, b = a ^ 1;
-        uint32_t* status = w.sort_status + (size_t)ps * w.sort_tiles * 256;
-        GS_TRY_LAUNCH(launch(next_pdl(), sort_pass_kernel(ps == 0, kpt, s->shape), (int)sort_tiles_of(n, kpt),
-                             kSortThreads, st, (const uint32_t*)w.keys[a], (const uint32_t*)(ps == 0 ? nullptr : w.idx[a]),
-                             w.keys[b], w.idx[b], n, 8 * ps, (const uint32_t*)(w.hist + 256 * ps), status,
-                             ctr + kCtrSort + ps, s->d_err));
-    }
-    count_launch(s, w.passes);
     w.final_keys = w.passes & 1;
-    stage_end(s, kStageSort, profile);
     const uint32_t* skey = w.keys[w.final_keys];
     const uint32_t* sidx = w.idx[w.final_keys];
-    stage_begin(s, kStageScan, profile);
-    GS_TRY_LAUNCH(launch(next_pdl(), meta_scan_kernel(s->shape.scan_lookback), (int)w.scan_tiles, kScanThreads, st,
-                         skey, n + 1,
-                         (const uint32_t*)(ctr + kCtrValid), w.depth, w.E, w.scan_status, ctr + kCtrScan,
-                         ctr + kCtrInternal, s->d_err));
-    count_launch(s);
-    stage_end(s, kStageScan, profile);
     MomIn mi{};
     if (w.quad) {  // exact moment sums: integer values in k_records, prefix in k_mom_scan, moments in k_nodes
         mi.bp = w.params;
@@ -1443,15 +1753,88 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     const bool heavy = w.heavy_flag && w.quad && (s->p.flags & GS_FLAG_GROUP_WALK) && n >= kHeavyMinParticles;
     HeavyOut ho{};
     if (heavy) ho = HeavyOut{w.amag, w.heavy_flag, w.heavy_list, ctr + kCtrHeavy, 0u};
-    stage_begin(s, kStageRecords, profile);
-    GS_TRY_LAUNCH(launch(next_pdl(), k_records, grid_for(n, 256), 256, st, skey, sidx, (const uint32_t*)w.E,
-                         (const uint32_t*)(ctr + kCtrValid), w.depth, (const float2*)s->pos[in],
-                         (const float*)s->mass[in], w.rec, w.skip, w.node_slot, w.cap, n, s->d_err, mi, ho));
+    if (small) {
+        SmallTree a{};
+        a.pos_in = s->pos[in];
+        a.mass_in = s->mass[in];
+        a.pos_out = s->pos[out];
+        a.mass_out = s->mass[out];
+        a.n = n;
+        a.bbox = bbox ? 1 : 0;
+        a.passes = w.passes;
+        a.D = w.depth;
+        a.counters = ctr;
+        a.params = w.params;
+        a.ext_in = bbox ? w.ext + 4 * in : nullptr;
+        a.ext_out = bbox ? w.ext + 4 * out : nullptr;
+        a.keys = w.keys[w.final_keys];
+        a.idx = w.idx[w.final_keys];
+        a.rec = w.rec;
+        a.skip = w.skip;
+        a.kids = w.kids;
+        a.nodeinfo = w.nodeinfo;
+        a.node_slot = w.node_slot;
+        a.levels = w.levels;
+        a.msum = w.msum;
+        a.safe = (s->p.flags & GS_FLAG_SAFE_RADIUS) ? 1 : 0;
+        a.links = w.quad || (s->p.flags & GS_FLAG_GROUP_WALK) ? 1 : 0;
+        a.cap = w.cap;
+        a.err = s->d_err;
+        a.mi = mi;
+        const auto run = [&](auto kernel, size_t bytes) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            return e != cudaSuccess ? e : launch_shared(next_pdl(), kernel, 1, kTreeThreads, (unsigned)bytes, st, a);
+        };
+        stage_begin(s, kStageRecords, profile);
+        GS_TRY_LAUNCH(n <= 2 * kTreeThreads   ? run(k_small_tree<2>, sizeof(TreeSmem<2>))
+                      : n <= 4 * kTreeThreads ? run(k_small_tree<4>, sizeof(TreeSmem<4>))
+                                              : run(k_small_tree<8>, sizeof(TreeSmem<8>)));
+        count_launch(s);
+    } else {
+        GS_TRY_LAUNCH(cudaMemsetAsync(w.zero_base, 0, w.zero_bytes, st));
+        stage_begin(s, kStageKeys, profile);
+        if (bbox) {  // the box from the extent carried with the input set
+            GS_TRY_LAUNCH(launch(next_pdl(), k_ext_keys, keygen_blocks(n), kKeyThreads, st, s->pos[in], s->mass[in],
+                                 s->pos[out], s->mass[out], n, w.keys[0], w.hist, w.passes, ctr + kCtrValid, w.params,
+                                 (const uint32_t*)(w.ext + 4 * in), w.ext + 4 * out, w.depth,
+                                 w.quad ? ctr + kCtrMaxMass : nullptr));
+        } else {
+            GS_TRY_LAUNCH(launch(next_pdl(), k_keygen, keygen_blocks(n), kKeyThreads, st, 0,
+                                 (const BHParams*)w.params, s->pos[in], s->mass[in], s->pos[out], s->mass[out], n,
+                                 w.keys[0], w.hist, w.passes, ctr + kCtrValid, w.quad ? ctr + kCtrMaxMass : nullptr));
+        }
+        count_launch(s);
+        stage_end(s, kStageKeys, profile);
+        stage_begin(s, kStageSort, profile);
+        const uint32_t kpt = sort_kpt(n, s->shape);
+        for (int ps = 0; ps < w.passes; ++ps) {
+            const int a = ps & 1, b = a ^ 1;
+            uint32_t* status = w.sort_status + (size_t)ps * w.sort_tiles * 256;
+            GS_TRY_LAUNCH(launch(next_pdl(), sort_pass_kernel(ps == 0, kpt, s->shape), (int)sort_tiles_of(n, kpt),
+                                 kSortThreads, st, (const uint32_t*)w.keys[a], (const uint32_t*)(ps == 0 ? nullptr : w.idx[a]),
+                                 w.keys[b], w.idx[b], n, 8 * ps, (const uint32_t*)(w.hist + 256 * ps), status,
+                                 ctr + kCtrSort + ps, s->d_err));
+        }
+        count_launch(s, w.passes);
+        stage_end(s, kStageSort, profile);
+        stage_begin(s, kStageScan, profile);
+        GS_TRY_LAUNCH(launch(next_pdl(), meta_scan_kernel(s->shape.scan_lookback), (int)w.scan_tiles, kScanThreads, st,
+                             skey, n + 1,
+                             (const uint32_t*)(ctr + kCtrValid), w.depth, w.E, w.scan_status, ctr + kCtrScan,
+                             ctr + kCtrInternal, s->d_err));
+        count_launch(s);
+        stage_end(s, kStageScan, profile);
+        stage_begin(s, kStageRecords, profile);
+        GS_TRY_LAUNCH(launch(next_pdl(), k_records, grid_for(n, 256), 256, st, skey, sidx, (const uint32_t*)w.E,
+                             (const uint32_t*)(ctr + kCtrValid), w.depth, (const float2*)s->pos[in],
+                             (const float*)s->mass[in], w.rec, w.skip, w.node_slot, w.cap, n, s->d_err, mi, ho));
+        count_launch(s);
+    }
     // Quadrupole mode without stage events: the moment prefix (k_mom_tiles, k_mom_scan)
     // and the node layout (k_nodes) read only what k_records and the scan wrote and write
     // disjoint buffers, so the prefix runs on the second stream beside k_nodes and
     // k_mom_nodes waits for both.
-    const bool fork = w.quad && pdl;
+    const bool fork = w.quad && pdl && !small;
     cudaStream_t mst = fork ? s->side : st;
     if (fork) {
         GS_TRY_LAUNCH(cudaEventRecord(s->fork_ev, st));
@@ -1464,11 +1847,13 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
                              (const uint32_t*)(ctr + kCtrValid), mi));
         count_launch(s, 2);
     }
-    GS_TRY_LAUNCH(launch(next_pdl(), k_nodes, grid_for(n, 256), 256, st, skey, (const uint32_t*)w.E,
-                         (const uint32_t*)(ctr + kCtrValid), w.depth, (const BHParams*)w.params,
-                         (const uint32_t*)w.node_slot, w.rec, w.skip, w.kids, w.nodeinfo, ctr + kCtrLevel, w.levels,
-                         n, w.cap, s->d_err, mi, w.quad, (s->p.flags & GS_FLAG_SAFE_RADIUS) ? 1 : 0));
-    count_launch(s, 2);
+    if (!small) {
+        GS_TRY_LAUNCH(launch(next_pdl(), k_nodes, grid_for(n, 256), 256, st, skey, (const uint32_t*)w.E,
+                             (const uint32_t*)(ctr + kCtrValid), w.depth, (const BHParams*)w.params,
+                             (const uint32_t*)w.node_slot, w.rec, w.skip, w.kids, w.nodeinfo, ctr + kCtrLevel, w.levels,
+                             n, w.cap, s->d_err, mi));
+        count_launch(s);
+    }
     if (fork) {  // the join: k_mom_nodes follows both streams with a plain launch
         GS_TRY_LAUNCH(cudaEventRecord(s->join_ev, mst));
         GS_TRY_LAUNCH(cudaStreamWaitEvent(st, s->join_ev, 0));
@@ -1483,25 +1868,15 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     }
     stage_end(s, kStageRecords, profile);
     stage_begin(s, kStageSums, profile);
-    if (!w.quad) {  // monopole moments, level by level (the quadrupole mode has them from k_nodes)
+    if (!w.quad && !small) {  // monopole moments, level by level (the quadrupole mode has them from k_nodes)
         const int safe = (s->p.flags & GS_FLAG_SAFE_RADIUS) ? 1 : 0;
         const int bb = bbox ? 1 : 0;
-        if (n <= kSmallSumsMax) {
-            GS_TRY_LAUNCH(cudaFuncSetAttribute(k_small_sums, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)sizeof(SmallSmem)));
-            GS_TRY_LAUNCH(launch_shared(next_pdl(), k_small_sums, 1, kSmallThreads, (unsigned)sizeof(SmallSmem), st,
-                                        (const uint32_t*)(ctr + kCtrValid), (const uint32_t*)(ctr + kCtrLevel),
-                                        (const uint32_t*)w.levels, n, skey, w.depth, w.rec, (const uint4*)w.kids,
-                                        (const uint2*)w.nodeinfo, w.msum, safe, bb, (const BHParams*)w.params,
-                                        (uint32_t)w.cap));
-        } else {
-            const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm
-                                                                                    : w.sums_per_sm;
-            GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, w.sms * per_sm, kCoopSumsThreads, st,
-                                      (const uint32_t*)(ctr + kCtrLevel), (const uint32_t*)w.levels, n, skey, w.depth,
-                                      w.rec, (const uint4*)w.kids, (const uint2*)w.nodeinfo, w.msum, safe, bb,
-                                      (const BHParams*)w.params, ctr + kCtrBarrier, s->d_err));
-        }
+        const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm
+                                                                                : w.sums_per_sm;
+        GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, w.sms * per_sm, kCoopSumsThreads, st,
+                                  (const uint32_t*)(ctr + kCtrLevel), (const uint32_t*)w.levels, n, skey, w.depth,
+                                  w.rec, (const uint4*)w.kids, (const uint2*)w.nodeinfo, w.msum, safe, bb,
+                                  (const BHParams*)w.params, ctr + kCtrBarrier, s->d_err));
         count_launch(s);
     }
     stage_end(s, kStageSums, profile);
@@ -1765,7 +2140,7 @@ __global__ void __launch_bounds__(256) kb_nodes(BatchArgs a) {
     const SysDesc& d = *bb.d;
     nodes_body(bb.blk, d.keys[d.passes & 1], d.E, d.counters + kCtrValid, d.depth, d.params, d.node_slot, d.rec,
                d.skip, d.kids, d.nodeinfo, d.counters + kCtrLevel, d.levels, d.n_al, d.cap, d.err,
-               batch_mom_in(d), d.quad, d.safe);
+               batch_mom_in(d));
 }
 
 __global__ void __launch_bounds__(256) kb_mom_nodes(BatchArgs a) {
