@@ -633,6 +633,7 @@ struct GroupSys {
     float alpha, floor2;
     uint32_t* ext;
     const uint8_t* heavy;
+    uint32_t tail = 0xffffffffu;  // blocks from here on take one group on both warps (WalkShape MIXED)
 };
 
 // The walk of a group: tests the records; flush(slot, nodes, runs, done) takes the lists,
@@ -1087,10 +1088,12 @@ __device__ __forceinline__ void force_pair_body(
 
 // The launch of a group-walk kernel: GROUPS groups per block, on one warp each or (SPLIT) two;
 // long or short lists (gs_shape).
-template <int GROUPS, bool SHORT, bool SPLIT>
+template <int GROUPS, bool SHORT, bool SPLIT, bool MIXED = false>
 struct WalkShape {
-    using Smem = typename std::conditional<SPLIT, GroupSmem<SHORT ? 31 : 63, SHORT ? 31 : 63, 2>,
-                                           GroupSmem<SHORT ? 64 : 128, SHORT ? 32 : 64, 1>>::type;
+    using SplitSmem = GroupSmem<SHORT ? 31 : 63, SHORT ? 31 : 63, 2>;
+    using Smem = typename std::conditional<SPLIT, SplitSmem, GroupSmem<SHORT ? 64 : 128, SHORT ? 32 : 64, 1>>::type;
+    static_assert(!MIXED || (GROUPS == 2 && !SPLIT), "a block's two warps take two groups or share one");
+    static constexpr bool kMixed = MIXED;
     static constexpr int kGroups = GROUPS, kThreads = GROUPS * (SPLIT ? 64 : 32);
     // resident blocks the registers are cut for: one warp per group at 96 registers a thread
     // (20 groups an SM), two at 128 (8 groups: N = 100,000, 161 us a step against 167 with 12 and 179 with 16)
@@ -1102,9 +1105,13 @@ struct WalkShape {
 // warps first walks costly groups together in the bytes of its one (SPLIT) or two groups.
 template <class SH, bool HEAVY>
 struct WalkSmem {
-    typename SH::Smem g[SH::kGroups];
+    union {
+        typename SH::Smem g[SH::kGroups];
+        typename SH::SplitSmem split;  // kMixed
+    };
     uint32_t ticket[SH::kThreads / 32];
     __device__ __forceinline__ typename SH::Smem& walk(int i) { return g[i]; }
+    __device__ __forceinline__ typename SH::SplitSmem& both() { return split; }
 };
 template <class SH>
 struct WalkSmem<SH, true> {
@@ -1164,8 +1171,15 @@ k_force_group(GroupSys y, const uint2* __restrict__ heavy_list, uint32_t* __rest
         for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.ticket[pair], pair)) < cnt;)
             force_pair_body<EXACT, COUNT>(y, heavy_list[u].y, pair, (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
     }
-    walk_init(sm.walk(walk), pair);
     uint32_t phase = 0;
+    if constexpr (SH::kMixed) {
+        if (blockIdx.x >= y.tail) {
+            walk_init(sm.both(), 0);
+            force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(y, y.tail + blockIdx.x, is_walker(), phase, sm.both());
+            return;
+        }
+    }
+    walk_init(sm.walk(walk), pair);
     force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(y, blockIdx.x * SH::kGroups + walk, !SH::kSplit || is_walker(), phase,
                                                    sm.walk(walk));
 }
@@ -1253,9 +1267,11 @@ using BatchGroupFn = void (*)(BatchArgs, uint32_t*, const uint2*, uint32_t*);
 // need two warps per block at least.
 template <bool EXACT, bool COUNT, class SH>
 GroupFn group_fn(bool quad, bool est, bool heavy) {
-    if (est) return k_force_group<EXACT, true, COUNT, true, SH, false>;
-    if constexpr (SH::kThreads >= 64)
-        if (heavy) return k_force_group<EXACT, true, COUNT, false, SH, true>;
+    if constexpr (!SH::kMixed) {
+        if (est) return k_force_group<EXACT, true, COUNT, true, SH, false>;
+        if constexpr (SH::kThreads >= 64)
+            if (heavy) return k_force_group<EXACT, true, COUNT, false, SH, true>;
+    }
     return quad ? k_force_group<EXACT, true, COUNT, false, SH, false>
                 : k_force_group<EXACT, false, COUNT, false, SH, false>;
 }
@@ -1270,12 +1286,13 @@ BatchGroupFn batch_group_fn(bool quad, bool est, bool heavy) {
 
 // fn(shape) with the shape launched for a request, its groups and threads per block.
 template <class Fn>
-auto with_shape(bool count, const gs_shape& sh, bool split, bool heavy, int* groups, int* threads, Fn&& fn) {
+auto with_shape(bool count, const gs_shape& sh, bool split, bool mixed, bool heavy, int* groups, int* threads, Fn&& fn) {
     const auto use = [&](auto shape) {
         *groups = decltype(shape)::kGroups;
         *threads = decltype(shape)::kThreads;
         return fn(shape);
     };
+    if (mixed) return use(WalkShape<2, false, false, true>{});
     if (count) return use(WalkShape<2, false, false>{});
     const uint32_t g = heavy && !split && sh.force_warps == 1 ? 2u : sh.force_warps;
     if (sh.force_short_lists) return split ? use(WalkShape<2, true, true>{}) : use(WalkShape<2, true, false>{});
@@ -1287,10 +1304,24 @@ auto with_shape(bool count, const gs_shape& sh, bool split, bool heavy, int* gro
 // Two warps per group where the launch's groups cannot fill the SMs on one warp each.
 constexpr uint32_t kSplitGroups = 152 * 14;
 
+// Larger launches: the last groups on two warps each, so that the chip does not end on whole
+// single-warp walks.  Five such groups an SM; eight where every group starts at once (3,040 on
+// one warp each).  Step with none and with these, relative criterion: 140,000 particles 236 and
+// 230 us, 150,000 223 and 197, 200,000 264 and 261; theta 0.35: 250,000 270 and 262, 450,000 398
+// and 384.  Not with warp pairs for costly groups, which are that launch's end whatever the last
+// groups do (five steps of 300,000 1.95 and 1.99 ms), nor by theta where every group starts at
+// once (its walks differ little: 180,000 1.17 and 1.20 ms).
+inline uint32_t tail_groups(uint32_t n_groups) { return n_groups <= 152 * kSinglePerSm ? 152 * 8 : 152 * 5; }
+inline bool walk_tail(const ForceLaunch& f, uint32_t n_groups, bool heavy) {
+    static_assert(kSplitGroups > 152 * 8, "some groups are left on one warp");
+    return n_groups > kSplitGroups && (f.amag ? !heavy : n_groups > 152 * kSinglePerSm) && !f.count && !f.estimate &&
+           f.shape.force_warps == 2 && !f.shape.force_short_lists;
+}
+
 template <bool EXACT>
-GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad, bool est, bool heavy, int* groups,
-                   int* threads) {
-    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
+GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool mixed, bool quad, bool est, bool heavy,
+                   int* groups, int* threads) {
+    return with_shape(count, sh, n_groups <= kSplitGroups, mixed, heavy, groups, threads, [&](auto s) {
         using SH = decltype(s);
         if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
             if (count) return group_fn<EXACT, true, SH>(quad, est, heavy);
@@ -1301,7 +1332,7 @@ GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad,
 template <bool EXACT>
 BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad, bool est, bool heavy,
                               int* groups, int* threads) {
-    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
+    return with_shape(count, sh, n_groups <= kSplitGroups, false, heavy, groups, threads, [&](auto s) {
         using SH = decltype(s);
         if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
             if (count) return batch_group_fn<EXACT, true, SH>(quad, est, heavy);
@@ -1332,11 +1363,16 @@ cudaError_t force_launch_impl(const ForceLaunch& f) {
     int groups = 2, threads = 64;
     const bool heavy = f.heavy && f.quad && !f.estimate;
     const uint32_t n_groups = f.n_al / kGroupSize;
-    GroupFn fn = pick_group<EXACT>(f.count, f.shape, n_groups, f.quad, f.estimate, heavy, &groups, &threads);
-    const int blocks = (int)((n_groups + groups - 1) / groups);
-    const GroupSys y{f.sidx, f.skey, f.counts, f.rec, f.skip, f.quad_m, f.kids, f.pos_in, f.vel_in, f.pos_out, f.vel_out,
+    const bool mixed = walk_tail(f, n_groups, heavy);
+    GroupFn fn = pick_group<EXACT>(f.count, f.shape, n_groups, mixed, f.quad, f.estimate, heavy, &groups, &threads);
+    int blocks = (int)((n_groups + groups - 1) / groups);
+    GroupSys y{f.sidx, f.skey, f.counts, f.rec, f.skip, f.quad_m, f.kids, f.pos_in, f.vel_in, f.pos_out, f.vel_out,
                      f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.err, f.amag, f.alpha, f.floor2,
                      f.ext, heavy ? f.heavy : nullptr};
+    if (mixed) {
+        y.tail = (n_groups - tail_groups(n_groups)) / 2;
+        blocks = (int)(n_groups - y.tail);
+    }
     return launch(f.pdl, fn, blocks, threads, f.st, y, heavy ? f.heavy_list : nullptr,
                   heavy ? f.heavy_work : nullptr);
 }
