@@ -46,7 +46,11 @@ struct RuleWindow {
 // and tests are made together (two records per packed instruction), and when all four are
 // accepted and follow one another (particle leaves) all four are summed at once; otherwise
 // the four are gone through in order with the distances at hand, as the rule does one by
-// one.  The sums take the records in the same order either way.
+// one.  After a round that left by an accepted node's skip before its last record the
+// next are taken singly until one is followed by its neighbour: a walk among accepted nodes
+// (the outskirts of a disk) tests few records in vain.  Force kernel, four always and so: 500k
+// spiral 172 and 162 us, 80,000 53.5 and 48.8, 20,000 galaxy 61.5 and 57.6, 3,000 24.6 and 22.6.
+// The sums take the records in the same order either way.
 // win: the warp's window, or with STAGED (win unused) the whole tree in shared memory at
 // s_rec / s_skip.
 template <bool EXACT, bool COUNT, bool FTZ, bool STAGED>
@@ -72,6 +76,7 @@ __device__ __forceinline__ void force_body(Blk blk, RuleWindow* win, const float
     float ax = 0.0f, ay = 0.0f;
     unsigned long long n_acc = 0, n_vis = 0;
     uint32_t base = 0, ind = 0;
+    bool single = false;
     if (!STAGED) {
         win->rec[lane] = rec[lane];
         win->skip[lane] = skip[lane];
@@ -87,6 +92,25 @@ __device__ __forceinline__ void force_body(Blk blk, RuleWindow* win, const float
         }
         const float4* q = STAGED ? s_rec + ind : win->rec + (ind - base);
         const uint32_t* sk = STAGED ? s_skip + ind : win->skip + (ind - base);
+        if (single) {
+            const float4 r0 = q[0];
+            const uint32_t step = sk[0];
+            const float dx = r0.x - p.x, dy = r0.y - p.y, d2 = fmaf(dx, dx, fmaf(dy, dy, eps2));
+            if (COUNT) ++n_vis;
+            if (__all_sync(0xffffffffu, !valid || r0.w <= d2 * theta2)) {
+                const float r = rule_inv_sqrt<EXACT, FTZ>(d2);
+                const float sc = ((r0.z * r) * r) * r;
+                ax = fmaf(dx, sc, ax);
+                ay = fmaf(dy, sc, ay);
+                if (COUNT) n_acc += valid;
+                ind += max(step, 1u);  // >= 1: the walk always advances
+                single = step > 1u;
+            } else {
+                ++ind;
+                single = false;
+            }
+            continue;
+        }
         const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3];
         const float2 dxa = sub2(make_float2(q0.x, q1.x), P), dya = sub2(make_float2(q0.y, q1.y), Q);
         const float2 dxb = sub2(make_float2(q2.x, q3.x), P), dyb = sub2(make_float2(q2.y, q3.y), Q);
@@ -113,16 +137,18 @@ __device__ __forceinline__ void force_body(Blk blk, RuleWindow* win, const float
                 n_vis += 4;
                 n_acc += valid ? 4 : 0;
             }
-            ind += 3u + max(sk3, 1u);  // >= 1: the walk always advances
+            ind += 3u + max(sk3, 1u);
             continue;
         }
         const float qm[4] = {q0.z, q1.z, q2.z, q3.z}, dd[4] = {da.x, da.y, db.x, db.y};
         const float dx[4] = {dxa.x, dxa.y, dxb.x, dxb.y}, dy[4] = {dya.x, dya.y, dyb.x, dyb.y};
         const uint32_t sks[4] = {sk0, sk1, sk2, sk3};
+        uint32_t used = 0;
         uint32_t next = 0;  // the next record of the rule's walk, from ind
 #pragma unroll
         for (uint32_t t = 0; t < 4; ++t) {
             if (next != t || t >= left) continue;  // uniform
+            ++used;
             if (COUNT) ++n_vis;
             if (__all_sync(0xffffffffu, ok[t])) {
                 const float r = rule_inv_sqrt<EXACT, FTZ>(dd[t]);
@@ -136,6 +162,7 @@ __device__ __forceinline__ void force_body(Blk blk, RuleWindow* win, const float
             }
         }
         ind += next;
+        single = used <= 3u && next > used;
     }
     if (COUNT) {
         for (int o = 16; o; o >>= 1) n_acc += __shfl_xor_sync(0xffffffffu, n_acc, o);
