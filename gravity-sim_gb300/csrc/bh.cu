@@ -1159,6 +1159,17 @@ __device__ __forceinline__ void top_sums_body(const uint32_t* __restrict__ level
 // block 0 with block barriers.  Each level's nodes are computed exactly as by the
 // per-level launches.
 constexpr int kCoopSumsThreads = 256;
+// Blocks of the launch, at most `resident`.  A level of a small system is a few nodes a thread
+// even in a few blocks, every block makes each of the barriers dearer, and the SMs that the
+// launch leaves free take the traversal's blocks early.  Step of the reference rule with 304
+// blocks and with these: 9,000 particles 123 and 102 us, 40,000 164 and 139, 60,000 138 and
+// 123, 100,000 222 and 207, 130,000 236 and 230, 200,000 and up the same within 0.5 %.  Caps of
+// 64, 128 or 152 blocks gained nothing there and cost up to 13 % at 250,000 to 300,000, where
+// they leave the traversal's blocks unevenly spread.
+inline int coop_sums_blocks(uint64_t n, int resident) {
+    const int fit = (int)std::max<uint64_t>(n / 2048, std::min<uint64_t>(n / 1024, 32));
+    return std::max(1, std::min(fit, resident));
+}
 
 __global__ void __launch_bounds__(kCoopSumsThreads, 2)
 k_coop_sums(const uint32_t* __restrict__ level_count, const uint32_t* __restrict__ levels, uint32_t n_al,
@@ -1873,7 +1884,7 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
         const int bb = bbox ? 1 : 0;
         const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm
                                                                                 : w.sums_per_sm;
-        GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, w.sms * per_sm, kCoopSumsThreads, st,
+        GS_TRY_LAUNCH(launch_coop(next_pdl(), k_coop_sums, coop_sums_blocks(n, w.sms * per_sm), kCoopSumsThreads, st,
                                   (const uint32_t*)(ctr + kCtrLevel), (const uint32_t*)w.levels, n, skey, w.depth,
                                   w.rec, (const uint4*)w.kids, (const uint2*)w.nodeinfo, w.msum, safe, bb,
                                   (const BHParams*)w.params, ctr + kCtrBarrier, s->d_err));
