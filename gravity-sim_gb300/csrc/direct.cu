@@ -7,7 +7,7 @@
 // positions and float2 pairs of masses: j-tiles start at multiples of 64) and broadcast to
 // the threads, which keep their targets in registers.  Each 64-wide tile is summed plainly
 // in FP32, and the tile partials are added with Kahan compensation.
-//   k_direct_small  (N <= 8192) 32 targets per block, the tiles split over its 16 warps and
+//   k_direct_small  (N <= 12,288) 32 targets per block, the tiles split over its 16 warps and
 //                   the warps' compensated sums added in shared memory
 //   k_direct_fast   (larger N) i-tiles of 128 threads with IPT targets each, j-chunks; every
 //                   block stores its compensated partial and the last block to finish an

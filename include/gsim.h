@@ -155,7 +155,8 @@ typedef struct gs_shape {
 } gs_shape;
 
 /* Statistics: stage times accumulate over steps since gs_reset_stats (GS_FLAG_PROFILE);
- * tree counts are those of the most recent step. */
+ * tree counts are those of the most recent step.  A small system's tree is built by one
+ * kernel, timed under records. */
 #define GS_STAGE_COUNT 8
 typedef struct gs_stats {
     uint64_t steps_done;
