@@ -49,7 +49,7 @@ struct RuleWindow {
 // one.  After a round that left by an accepted node's skip before its last record the
 // next are taken singly until one is followed by its neighbour: a walk among accepted nodes
 // (the outskirts of a disk) tests few records in vain.  Force kernel, four always and so: 500k
-// spiral 172 and 162 us, 80,000 53.5 and 48.8, 20,000 galaxy 61.5 and 57.6, 3,000 24.6 and 22.6.
+// spiral 172 and 162 us, 80,000 53.5 and 48.5, 20,000 galaxy 61.5 and 57.6, 3,000 24.6 and 22.8.
 // The sums take the records in the same order either way.
 // win: the warp's window, or with STAGED (win unused) the whole tree in shared memory at
 // s_rec / s_skip.
