@@ -328,12 +328,14 @@ k_direct_small(const float2* __restrict__ pos, const float2* __restrict__ vel, c
 // then the residual x - g^2, exact in an FMA, gives the rounded root s = g + (x - g^2) h, and two
 // steps r += (1 - s r) r from r = 2 h the rounded reciprocal (one leaves two mantissas, whose
 // reciprocals lie 5e-8 of a unit from a rounding boundary, one unit off).  No step overflows
-// or loses bits to underflow for x in [2^-100, 2^100].  A root of all-ones mantissa, the case
-// Markstein's theorem on reciprocals leaves out, comes from an x of all-ones mantissa.  Those,
-// and an x outside the range (a zero, a NaN, an overflowed distance), go to the library
-// functions; compared with them on the GPU, every float from 0 to infinity is equal.  In packed f32x2
-// form the chain is 6.5 issues a value; the library's root and reciprocal carry their own
-// range checks and branches, most of the 47 instructions that a factor cost.
+// or loses bits to underflow for x in [2^-100, 2^100].  Markstein's theorem on reciprocals leaves
+// out a root of all-ones mantissa: r stays 2^-k, its residual half a unit that rounds away.  Such
+// a root comes from the two floats just below a power of 4, mantissas 0x7ffffe and 0x7fffff.
+// Those, and an x outside the range (a zero, a NaN, an overflowed distance), go to the library
+// functions; with them every mantissa of both exponent parities gives the library's bits, for any
+// estimate y within two units of the root's reciprocal.  In packed f32x2 form the chain is 6.5
+// issues a value; the library's root and reciprocal carry their own range checks and branches,
+// most of the 47 instructions that a factor cost.
 __device__ __forceinline__ float2 ref_inv_sqrt2(float2 x) {
     const float2 y = make_float2(direct_rsqrt<true>(x.x), direct_rsqrt<true>(x.y));
     float2 g = mul2(x, y), h = mul2(y, make_float2(0.5f, 0.5f));
@@ -345,7 +347,7 @@ __device__ __forceinline__ float2 ref_inv_sqrt2(float2 x) {
     const float2 r = add2(h, h), r1 = fma2(fma2(ns, r, one), r, r);
     float2 v = fma2(fma2(ns, r1, one), r1, r1);
     const float lo = 7.888609052e-31f, hi = 1.267650600e30f;  // 2^-100, 2^100
-    const uint32_t ones = 0x7fffffu;
+    const uint32_t ones = 0x7ffffeu;  // the last mantissa bit is free
     if (!(x.x >= lo && x.x <= hi && x.y >= lo && x.y <= hi) || (__float_as_uint(x.x) & ones) == ones ||
         (__float_as_uint(x.y) & ones) == ones) {
         v.x = __frcp_rn(__fsqrt_rn(x.x));
