@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "bh_common.cuh"
+#include "pair_loop.h"
 
 namespace gsim {
 namespace {
@@ -1136,7 +1137,7 @@ struct WalkSmem {
         typename SH::Smem g[SH::kGroups];
         typename SH::SplitSmem split;  // kMixed
     };
-    uint32_t ticket[SH::kThreads / 32];
+    PairTurn turn[(SH::kThreads + 63) / 64];
     __device__ __forceinline__ typename SH::Smem& walk(int i) { return g[i]; }
     __device__ __forceinline__ typename SH::SplitSmem& both() { return split; }
 };
@@ -1147,7 +1148,7 @@ struct WalkSmem<SH, true> {
         typename SH::Smem g[kPer];
         PairSmem pair;
     } p[SH::kThreads / 64];
-    uint32_t ticket[SH::kThreads / 32];
+    PairTurn turn[(SH::kThreads + 63) / 64];
     __device__ __forceinline__ typename SH::Smem& walk(int i) { return p[i / kPer].g[i % kPer]; }
 };
 
@@ -1195,7 +1196,7 @@ k_force_group(GroupSys y, const uint2* __restrict__ heavy_list, uint32_t* __rest
     if constexpr (HEAVY) {
         static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
         const uint32_t cnt = hwork[0];
-        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.ticket[pair], pair)) < cnt;)
+        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.turn[pair].unit, pair)) < cnt;)
             force_pair_body<EXACT, COUNT>(y, heavy_list[u].y, pair, (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
     }
     uint32_t phase = 0;
@@ -1232,7 +1233,7 @@ kb_force_group(BatchArgs a, uint32_t* __restrict__ work, const uint2* __restrict
     if constexpr (HEAVY) {
         static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
         const uint32_t cnt = hwork[0];
-        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.ticket[pair], pair)) < cnt;) {
+        for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.turn[pair].unit, pair)) < cnt;) {
             const uint2 e = heavy_list[u];
             const SysDesc& d = a.descs[e.x];
             const int in = (int)((d.parity + a.step) & 1u);
@@ -1240,17 +1241,21 @@ kb_force_group(BatchArgs a, uint32_t* __restrict__ work, const uint2* __restrict
                                           (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
         }
     }
-    walk_init(sm.walk(walk), pair);
+    if (SH::kSplit && (threadIdx.x & 63u) == 0) sm.turn[pair].failed = 0u;
+    walk_init(sm.walk(walk), pair);  // SPLIT: with a barrier of the pair
     const uint32_t total = __ldg(&a.first[a.nsys]);
     const bool walker = !SH::kSplit || is_walker();
     uint32_t phase = 0;
-    for (;;) {
-        const uint32_t u = SH::kSplit ? pair_ticket(work, total, sm.ticket[pair], pair) : warp_ticket(work, total);
-        if (u >= total) break;
+    const auto group = [&](uint32_t u) {
         const BatchBlock bb = batch_block(a, u);
-        if (!force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(batch_group_sys(*bb.d, bb.in, bb.out, HEAVY), bb.blk.id,
-                                                            walker, phase, sm.walk(walk)))
-            break;
+        return force_group_body<EXACT, QUAD, COUNT, ESTIMATE>(batch_group_sys(*bb.d, bb.in, bb.out, HEAVY), bb.blk.id,
+                                                              walker, phase, sm.walk(walk));
+    };
+    if constexpr (SH::kSplit) {
+        pair_loop(sm.turn[pair], (threadIdx.x & 63u) == 0, total,
+                  [&] { return __ldcg(work) < total ? atomicAdd(work, 1u) : total; }, [&] { pair_sync(pair); }, group);
+    } else {  // no walk of one warp waits for another
+        for (uint32_t u; (u = warp_ticket(work, total)) < total;) group(u);
     }
 }
 
