@@ -1646,7 +1646,14 @@ void bh_carve(gs_sim* s) {
     // 30-bit keys), 20-bit keys + removal bit in the fixed box (3 passes)
     w.passes = bbox ? (2 * w.depth + 7) / 8 : 3;
     w.cap = bh_capacity(w.depth, n);
-    w.sort_tiles = sort_tiles_of(n, n <= kSortSmallMax ? 4 : 8);  // status for the smallest tiles
+    w.sort_tiles = sort_tiles_of(n, 8);  // status for the smallest tiles of a shape
+    // A small system sorted alone has up to twice as many: the rest of their status, 2 n + 4096
+    // bytes at most and none below 1,025 particles, is the tail of node_slot, which is carved
+    // right before, is larger and is not read before k_records, after the sort, has written it.
+    // (Statuses of their own would be up to 0.7 % of the footprint and double the sort status
+    // that a batch, in tiles of its shape, clears for the system.)
+    w.sort_tiles_alone = n <= kSortSmallMax ? sort_tiles_of(n, 4) : w.sort_tiles;
+    w.sort_extra = (size_t)w.passes * (w.sort_tiles_alone - w.sort_tiles) * 256 * sizeof(uint32_t);
     w.scan_tiles = (uint32_t)((n + 1 + kScanTile - 1) / kScanTile);
     for (int b = 0; b < 2; ++b) {
         sim_carve(s, (void**)&w.keys[b], n * sizeof(uint32_t));
@@ -1661,7 +1668,6 @@ void bh_carve(gs_sim* s) {
     if (!(s->p.flags & GS_FLAG_QUADRUPOLE))
         sim_carve(s, (void**)&w.levels, (size_t)level_off(w.depth + 1, (uint32_t)n) * sizeof(uint32_t));
     sim_carve(s, (void**)&w.nodeinfo, w.cap * sizeof(uint2));
-    sim_carve(s, (void**)&w.node_slot, w.cap * sizeof(uint32_t));
     w.quad = nullptr;
     w.mom_q = nullptr;
     w.mom_prefix = nullptr;
@@ -1688,18 +1694,19 @@ void bh_carve(gs_sim* s) {
     if (bbox) sim_carve(s, (void**)&w.ext, 8 * sizeof(uint32_t));
     sim_carve(s, (void**)&w.bbox_part, kBBoxBlocks * 4 * sizeof(float));
     sim_carve(s, (void**)&w.params, sizeof(BHParams));
-    // one block cleared per step: hist | counters | sort status | scan status
+    // one block cleared per step: sort status | hist | counters | scan status, behind node_slot
+    const size_t sort_b = (size_t)w.passes * w.sort_tiles * 256 * sizeof(uint32_t);
     const size_t hist_b = 4 * 256 * sizeof(uint32_t);
     const size_t ctr_b = kCtrCount * sizeof(uint32_t);
-    const size_t sort_b = (size_t)w.passes * w.sort_tiles * 256 * sizeof(uint32_t);
     const size_t scan_b = (size_t)w.scan_tiles * sizeof(uint32_t);
-    w.zero_bytes = hist_b + ctr_b + sort_b + scan_b;
+    w.zero_bytes = sort_b + hist_b + ctr_b + scan_b;
+    sim_carve(s, (void**)&w.node_slot, w.cap * sizeof(uint32_t));
     sim_carve(s, &w.zero_base, w.zero_bytes);
     char* zb = (char*)w.zero_base;
-    w.hist = zb ? (uint32_t*)zb : nullptr;
-    w.counters = zb ? (uint32_t*)(zb + hist_b) : nullptr;
-    w.sort_status = zb ? (uint32_t*)(zb + hist_b + ctr_b) : nullptr;
-    w.scan_status = zb ? (uint32_t*)(zb + hist_b + ctr_b + sort_b) : nullptr;
+    w.sort_status = zb ? (uint32_t*)zb : nullptr;
+    w.hist = zb ? (uint32_t*)(zb + sort_b) : nullptr;
+    w.counters = zb ? (uint32_t*)(zb + sort_b + hist_b) : nullptr;
+    w.scan_status = zb ? (uint32_t*)(zb + sort_b + hist_b + ctr_b) : nullptr;
 }
 
 // Initial contents: everything a debug read of a never-built tree could see is zero, the
@@ -1802,7 +1809,8 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
                                               : run(k_small_tree<8>, sizeof(TreeSmem<8>)));
         count_launch(s);
     } else {
-        GS_TRY_LAUNCH(cudaMemsetAsync(w.zero_base, 0, w.zero_bytes, st));
+        char* zero = (char*)w.zero_base - w.sort_extra;  // from the sort status of a system alone on
+        GS_TRY_LAUNCH(cudaMemsetAsync(zero, 0, w.zero_bytes + w.sort_extra, st));
         stage_begin(s, kStageKeys, profile);
         if (bbox) {  // the box from the extent carried with the input set
             GS_TRY_LAUNCH(launch(next_pdl(), k_ext_keys, keygen_blocks(n), kKeyThreads, st, s->pos[in], s->mass[in],
@@ -1820,7 +1828,7 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
         const uint32_t kpt = sort_kpt(n, s->shape);
         for (int ps = 0; ps < w.passes; ++ps) {
             const int a = ps & 1, b = a ^ 1;
-            uint32_t* status = w.sort_status + (size_t)ps * w.sort_tiles * 256;
+            uint32_t* status = (uint32_t*)zero + (size_t)ps * w.sort_tiles_alone * 256;
             GS_TRY_LAUNCH(launch(next_pdl(), sort_pass_kernel(ps == 0, kpt, s->shape), (int)sort_tiles_of(n, kpt),
                                  kSortThreads, st, (const uint32_t*)w.keys[a], (const uint32_t*)(ps == 0 ? nullptr : w.idx[a]),
                                  w.keys[b], w.idx[b], n, 8 * ps, (const uint32_t*)(w.hist + 256 * ps), status,

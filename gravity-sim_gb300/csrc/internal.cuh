@@ -115,7 +115,7 @@ struct BHWork {
     uint32_t* keys[2] = {nullptr, nullptr};
     uint32_t* idx[2] = {nullptr, nullptr};
     uint32_t* hist = nullptr;          // [4][256] digit counts
-    uint32_t* sort_status = nullptr;   // [passes][tiles][256]
+    uint32_t* sort_status = nullptr;   // [passes][sort_tiles][256]
     uint32_t* counters = nullptr;      // [0..3] sort tile tickets, [4] scan ticket, [5] bbox ticket,
                                        // [6] valid count, [7] internal count, [8..13] interaction,
                                        // test and node counts (3 x u64), [16..31] nodes per level
@@ -144,6 +144,8 @@ struct BHWork {
     float* bbox_part = nullptr;        // [blocks][4]
     BHParams* params = nullptr;        // device
     uint32_t sort_tiles = 0, scan_tiles = 0;
+    uint32_t sort_tiles_alone = 0;     // radix tiles of the system sorted alone, at most
+    size_t sort_extra = 0;             // bytes of their status in front of sort_status
     int final_keys = 0;                // which keys/idx buffer holds the sorted result
     size_t zero_bytes = 0;             // bytes of the contiguous block cleared each step
     void* zero_base = nullptr;
