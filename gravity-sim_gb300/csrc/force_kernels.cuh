@@ -1129,8 +1129,8 @@ struct WalkShape {
     static constexpr bool kSplit = SPLIT;
 };
 
-// Shared memory of a block; with HEAVY (the main pass of the relative criterion) each pair of
-// warps first walks costly groups together in the bytes of its one (SPLIT) or two groups.
+// Shared memory of a block; with HEAVY (the main pass of the relative criterion, groups on one
+// warp each) each pair of warps first walks costly groups together in the bytes of its two groups.
 template <class SH, bool HEAVY>
 struct WalkSmem {
     union {
@@ -1143,13 +1143,13 @@ struct WalkSmem {
 };
 template <class SH>
 struct WalkSmem<SH, true> {
-    static constexpr int kPer = SH::kSplit ? 1 : 2;  // groups per pair of warps
+    static_assert(!SH::kSplit && SH::kThreads % 64 == 0, "whole pairs of warps, a group each");
     union Pair {
-        typename SH::Smem g[kPer];
+        typename SH::Smem g[2];
         PairSmem pair;
     } p[SH::kThreads / 64];
-    PairTurn turn[(SH::kThreads + 63) / 64];
-    __device__ __forceinline__ typename SH::Smem& walk(int i) { return p[i / kPer].g[i % kPer]; }
+    PairTurn turn[SH::kThreads / 64];
+    __device__ __forceinline__ typename SH::Smem& walk(int i) { return p[i / 2].g[i % 2]; }
 };
 
 // The next value of a counter below cnt for both warps of a pair, or a value >= cnt when none
@@ -1194,7 +1194,7 @@ k_force_group(GroupSys y, const uint2* __restrict__ heavy_list, uint32_t* __rest
     pdl_enter();
     const int pair = (int)(threadIdx.x >> 6), walk = SH::kSplit ? pair : (int)(threadIdx.x >> 5);
     if constexpr (HEAVY) {
-        static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
+        static_assert(QUAD && !ESTIMATE, "warp pairs walk costly groups of the relative main pass");
         const uint32_t cnt = hwork[0];
         for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.turn[pair].unit, pair)) < cnt;)
             force_pair_body<EXACT, COUNT>(y, heavy_list[u].y, pair, (int)((threadIdx.x >> 5) & 1u), sm.p[pair].pair);
@@ -1231,7 +1231,7 @@ kb_force_group(BatchArgs a, uint32_t* __restrict__ work, const uint2* __restrict
     pdl_enter();
     const int pair = (int)(threadIdx.x >> 6), walk = SH::kSplit ? pair : (int)(threadIdx.x >> 5);
     if constexpr (HEAVY) {
-        static_assert(QUAD && !ESTIMATE && SH::kThreads % 64 == 0, "warp pairs walk costly groups of the relative main pass");
+        static_assert(QUAD && !ESTIMATE, "warp pairs walk costly groups of the relative main pass");
         const uint32_t cnt = hwork[0];
         for (uint32_t u; (u = pair_ticket(hwork + 1, cnt, sm.turn[pair].unit, pair)) < cnt;) {
             const uint2 e = heavy_list[u];
@@ -1296,12 +1296,13 @@ using BatchGroupFn = void (*)(BatchArgs, uint32_t*, const uint2*, uint32_t*);
 
 // The group-walk kernel of one shape (counting variants: the default shape only); heavy:
 // the main pass with warp pairs for costly groups (quadrupoles, relative criterion), which
-// need two warps per block at least.
+// need two warps per block at least, and have them: only systems above kSplitGroups have
+// costly groups.
 template <bool EXACT, bool COUNT, class SH>
 GroupFn group_fn(bool quad, bool est, bool heavy) {
     if constexpr (!SH::kMixed) {
         if (est) return k_force_group<EXACT, true, COUNT, true, SH, false>;
-        if constexpr (SH::kThreads >= 64)
+        if constexpr (SH::kThreads >= 64 && !SH::kSplit)
             if (heavy) return k_force_group<EXACT, true, COUNT, false, SH, true>;
     }
     return quad ? k_force_group<EXACT, true, COUNT, false, SH, false>
@@ -1310,7 +1311,7 @@ GroupFn group_fn(bool quad, bool est, bool heavy) {
 template <bool EXACT, bool COUNT, class SH>
 BatchGroupFn batch_group_fn(bool quad, bool est, bool heavy) {
     if (est) return kb_force_group<EXACT, true, COUNT, true, SH, false>;
-    if constexpr (SH::kThreads >= 64)
+    if constexpr (SH::kThreads >= 64 && !SH::kSplit)
         if (heavy) return kb_force_group<EXACT, true, COUNT, false, SH, true>;
     return quad ? kb_force_group<EXACT, true, COUNT, false, SH, false>
                 : kb_force_group<EXACT, false, COUNT, false, SH, false>;
@@ -1318,15 +1319,14 @@ BatchGroupFn batch_group_fn(bool quad, bool est, bool heavy) {
 
 // fn(shape) with the shape launched for a request, its groups and threads per block.
 template <class Fn>
-auto with_shape(bool count, const gs_shape& sh, bool split, bool mixed, bool heavy, int* groups, int* threads, Fn&& fn) {
+auto with_shape(bool count, const gs_shape& sh, bool split, bool heavy, int* groups, int* threads, Fn&& fn) {
     const auto use = [&](auto shape) {
         *groups = decltype(shape)::kGroups;
         *threads = decltype(shape)::kThreads;
         return fn(shape);
     };
-    if (mixed) return use(WalkShape<2, false, false, true>{});
     if (count) return use(WalkShape<2, false, false>{});
-    const uint32_t g = heavy && !split && sh.force_warps == 1 ? 2u : sh.force_warps;
+    const uint32_t g = heavy && sh.force_warps == 1 ? 2u : sh.force_warps;
     if (sh.force_short_lists) return split ? use(WalkShape<2, true, true>{}) : use(WalkShape<2, true, false>{});
     if (g == 1) return split ? use(WalkShape<1, false, true>{}) : use(WalkShape<1, false, false>{});
     if (g == 4) return split ? use(WalkShape<4, false, true>{}) : use(WalkShape<4, false, false>{});
@@ -1335,6 +1335,7 @@ auto with_shape(bool count, const gs_shape& sh, bool split, bool mixed, bool hea
 
 // Two warps per group where the launch's groups cannot fill the SMs on one warp each.
 constexpr uint32_t kSplitGroups = 152 * 14;
+static_assert(kHeavyMinParticles / kGroupSize > kSplitGroups, "costly groups only where every group has one warp");
 
 // Larger launches: the last groups on two warps each, so that the chip does not end on whole
 // single-warp walks.  Five such groups an SM; eight where every group starts at once (3,040 on
@@ -1353,7 +1354,13 @@ inline bool walk_tail(const ForceLaunch& f, uint32_t n_groups, bool heavy) {
 template <bool EXACT>
 GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool mixed, bool quad, bool est, bool heavy,
                    int* groups, int* threads) {
-    return with_shape(count, sh, n_groups <= kSplitGroups, mixed, heavy, groups, threads, [&](auto s) {
+    if (mixed) {
+        using SH = WalkShape<2, false, false, true>;
+        *groups = SH::kGroups;
+        *threads = SH::kThreads;
+        return group_fn<EXACT, false, SH>(quad, est, heavy);
+    }
+    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
         using SH = decltype(s);
         if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
             if (count) return group_fn<EXACT, true, SH>(quad, est, heavy);
@@ -1364,7 +1371,7 @@ GroupFn pick_group(bool count, const gs_shape& sh, uint32_t n_groups, bool mixed
 template <bool EXACT>
 BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, uint32_t n_groups, bool quad, bool est, bool heavy,
                               int* groups, int* threads) {
-    return with_shape(count, sh, n_groups <= kSplitGroups, false, heavy, groups, threads, [&](auto s) {
+    return with_shape(count, sh, n_groups <= kSplitGroups, heavy, groups, threads, [&](auto s) {
         using SH = decltype(s);
         if constexpr (std::is_same<SH, WalkShape<2, false, false>>::value)
             if (count) return batch_group_fn<EXACT, true, SH>(quad, est, heavy);
@@ -1375,22 +1382,25 @@ BatchGroupFn pick_batch_group(bool count, const gs_shape& sh, uint32_t n_groups,
 template <bool EXACT>
 cudaError_t force_launch_impl(const ForceLaunch& f) {
     if (!f.group) {  // the reference's warp-vote walk
-        const bool ftz = EXACT || rule_ftz(f.eps2);
-        const int blocks = (int)((f.n_al / 32 + kForceWarps - 1) / kForceWarps);
-        if (f.n_al <= kRuleStagedMax) {
-            auto fn = f.count ? (ftz ? k_force_staged<EXACT, true, true> : k_force_staged<EXACT, true, false>)
-                              : (ftz ? k_force_staged<EXACT, false, true> : k_force_staged<EXACT, false, false>);
-            const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)sizeof(RuleTree));
-            if (e != cudaSuccess) return e;
-            return launch_shared(f.pdl, fn, blocks, kForceWarps * 32, (unsigned)sizeof(RuleTree), f.st, f.sidx,
-                                 f.counts, f.rec, f.skip, f.pos_in, f.vel_in, f.pos_out, f.vel_out, f.acc, f.n_al,
-                                 f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
-        }
-        auto fn = f.count ? (ftz ? k_force<EXACT, true, true> : k_force<EXACT, true, false>)
-                          : (ftz ? k_force<EXACT, false, true> : k_force<EXACT, false, false>);
-        return launch(f.pdl, fn, blocks, kForceWarps * 32, f.st, f.sidx, f.counts, f.rec, f.skip, f.pos_in, f.vel_in,
-                      f.pos_out, f.vel_out, f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
+        const auto run = [&](auto ftz) {
+            constexpr bool kFtz = decltype(ftz)::value;
+            const int blocks = (int)((f.n_al / 32 + kForceWarps - 1) / kForceWarps);
+            if (f.n_al <= kRuleStagedMax) {
+                auto fn = f.count ? k_force_staged<EXACT, true, kFtz> : k_force_staged<EXACT, false, kFtz>;
+                const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           (int)sizeof(RuleTree));
+                if (e != cudaSuccess) return e;
+                return launch_shared(f.pdl, fn, blocks, kForceWarps * 32, (unsigned)sizeof(RuleTree), f.st, f.sidx,
+                                     f.counts, f.rec, f.skip, f.pos_in, f.vel_in, f.pos_out, f.vel_out, f.acc, f.n_al,
+                                     f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
+            }
+            return launch(f.pdl, f.count ? k_force<EXACT, true, kFtz> : k_force<EXACT, false, kFtz>, blocks,
+                          kForceWarps * 32, f.st, f.sidx, f.counts, f.rec, f.skip, f.pos_in, f.vel_in, f.pos_out,
+                          f.vel_out, f.acc, f.n_al, f.eps2, f.theta2, f.k, f.hdt, f.cap, f.stat, f.ext);
+        };
+        if constexpr (!EXACT)
+            if (!rule_ftz(f.eps2)) return run(std::false_type{});
+        return run(std::true_type{});
     }
     int groups = 2, threads = 64;
     const bool heavy = f.heavy && f.quad && !f.estimate;
