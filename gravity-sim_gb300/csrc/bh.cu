@@ -1736,6 +1736,17 @@ cudaError_t bh_init(gs_sim* s) {
     return e;
 }
 
+static bool tree_small(uint64_t n_al, bool quad) { return n_al <= (quad ? kTreeSmallQuadMax : kTreeSmallMax); }
+
+ShapeUse bh_shape_use(const gs_params* p, uint64_t n_al, int sms) {
+    ShapeUse u;
+    const bool quad = (p->flags & GS_FLAG_QUADRUPOLE) != 0;
+    u.lookbacks = !tree_small(n_al, quad);
+    u.sort_tile = u.lookbacks && n_al > kSortSmallMax;
+    u.moments = u.lookbacks && !quad && coop_sums_blocks(n_al, sms) != coop_sums_blocks(n_al, 2 * sms);
+    return u;
+}
+
 cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     BHWork& w = s->bh;
     cudaStream_t st = s->stream;
@@ -1743,7 +1754,7 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     const bool bbox = s->p.box_mode == GS_BOX_BOUNDING;
     uint32_t* ctr = w.counters;
     // one block from the keys to the node layout and the monopole moments
-    const bool small = n <= (w.quad ? kTreeSmallQuadMax : kTreeSmallMax);
+    const bool small = tree_small(n, w.quad != nullptr);
     // programmatic launches everywhere except right after the memset, and not while
     // stage events sit between the launches
     const bool pdl = !profile;

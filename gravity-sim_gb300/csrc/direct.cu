@@ -780,6 +780,12 @@ static DirectGrid pick_grid(uint64_t n_al, uint32_t blocks_per_sm, uint32_t max_
 
 static int shape_ipt(const gs_shape& sh) { return sh.direct_targets == 4 ? 4 : 2; }
 
+ShapeUse direct_shape_use(const gs_params* p, uint64_t n_al) {
+    ShapeUse u;
+    u.direct = p->math_mode != GS_MATH_REFERENCE && n_al > kDirectSmallMax;
+    return u;
+}
+
 // Lays the j-chunk partials and tickets out in the system's slab (sizing pass: counts), for
 // the j-split of the creation shape.  direct_max_chunks keeps gs_set_shape's limit: a shape
 // may ask for no finer split than one laid out by pick_chunks would hold.

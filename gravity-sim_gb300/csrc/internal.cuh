@@ -293,6 +293,12 @@ gs_status cuda_fail(cudaError_t e, const char* what);
 bool shape_valid(const gs_shape& sh, std::string* why);
 void shape_for(const gs_params* p, uint64_t n, gs_shape* out);
 void batch_shape_for(const gs_params* p, uint64_t total, gs_shape* out);
+// Which fields of its launch shape the step of a system alone depends on at this size.
+struct ShapeUse {
+    bool sort_tile = false, lookbacks = false, moments = false, direct = false;
+};
+ShapeUse bh_shape_use(const gs_params* p, uint64_t n_al, int sms);
+ShapeUse direct_shape_use(const gs_params* p, uint64_t n_al);
 // The parameters and total particles a batch's tuned-table entry is keyed by.
 gs_status batch_key(gs_batch* b, gs_params* params, uint64_t* total);
 

@@ -7,6 +7,9 @@
 // and the tuner measures which values are fastest for a workload on this device:
 //   - coordinate descent from the defaults: each knob in turn takes each of its values with
 //     the others at their best so far, and keeps the fastest;
+//   - a field that the system's kernels do not read at this size is timed like the others but
+//     keeps its default: it could only win by noise, and the table's entry also serves the other
+//     sizes of its bucket, where the field may count;
 //   - a candidate's time is the median of `steps` device-timed steps (CUDA events on the
 //     system's stream), each after a 256 MiB write that flushes L2, after 3 warm steps;
 //   - winners are kept in a process-wide table keyed by device, algorithm, box mode, key
@@ -225,22 +228,23 @@ gs_status time_steps(cudaStream_t st, Flush& fl, uint32_t steps, Run run, double
 struct Knob {
     int field;                    // index into shape_field, or -1: the (warps, short lists) pair
     std::vector<uint32_t> values;
+    bool used = true;             // the workload's kernels depend on the field
 };
 
 // quadrupole mode: the moments come from exact sums (no cooperative moments launch), so
 // the moments grid is not a knob
-std::vector<Knob> knobs_for(int algorithm, bool group_walk, bool quadrupole) {
+std::vector<Knob> knobs_for(int algorithm, bool group_walk, bool quadrupole, const ShapeUse& use) {
     std::vector<Knob> k;
     if (algorithm == GS_DIRECT_SUM) {
-        k.push_back({5, {2, 4}});
-        k.push_back({6, {4, 8, 12, 16, 24}});
+        k.push_back({5, {2, 4}, use.direct});
+        k.push_back({6, {4, 8, 12, 16, 24}, use.direct});
         return k;
     }
-    k.push_back({0, {8, 16}});
-    k.push_back({1, {8, 16, 32}});
-    k.push_back({2, {32, 64, 128}});
+    k.push_back({0, {8, 16}, use.sort_tile});
+    k.push_back({1, {8, 16, 32}, use.lookbacks});
+    k.push_back({2, {32, 64, 128}, use.lookbacks});
     if (group_walk) k.push_back({-1, {10, 20, 21, 40}});  // warps * 10 + short lists
-    if (!quadrupole) k.push_back({7, {1, 2}});
+    if (!quadrupole) k.push_back({7, {1, 2}, use.moments});
     if (algorithm == kAlgoBatch) k.push_back({5, {2, 4}});  // the batch's direct-sum members
     return k;
 }
@@ -277,7 +281,7 @@ gs_status descend(const std::vector<Knob>& knobs, Measure measure, gs_tune_resul
             if (r == GS_ERR_CAPACITY) continue;
             if (r != GS_OK) return r;
             ++out->candidates;
-            if (ms < best_ms) {
+            if (k.used && ms < best_ms) {
                 best_ms = ms;
                 best = c;
             }
@@ -372,7 +376,11 @@ gs_status gs_tune_shape(const gs_params* params, uint64_t n, int32_t generator, 
         if (st != GS_OK) return st;
     }
     std::memset(out, 0, sizeof *out);
-    st = descend(knobs_for(p.algorithm, (p.flags & GS_FLAG_GROUP_WALK) != 0, (p.flags & GS_FLAG_QUADRUPOLE) != 0),
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
+    const uint64_t n_al = (n + kAlignment - 1) / kAlignment * kAlignment;
+    const ShapeUse use = bh ? bh_shape_use(&p, n_al, sms) : direct_shape_use(&p, n_al);
+    st = descend(knobs_for(p.algorithm, (p.flags & GS_FLAG_GROUP_WALK) != 0, (p.flags & GS_FLAG_QUADRUPOLE) != 0, use),
                  measure, out);
     if (sim) gs_destroy(sim);
     if (st != GS_OK) return st;
@@ -412,8 +420,10 @@ gs_status gs_tune_batch_shape(gs_batch* b, uint32_t steps, const char* cache_pat
         return time_steps(bs, fl, steps, [&]() { return gs_batch_run(b, 1); }, ms);
     };
     std::memset(out, 0, sizeof *out);
+    ShapeUse use;  // the batched kernels take every field at every size
+    use.sort_tile = use.lookbacks = use.moments = use.direct = true;
     st = descend(knobs_for(kAlgoBatch, (key_params.flags & GS_FLAG_GROUP_WALK) != 0,
-                           (key_params.flags & GS_FLAG_QUADRUPOLE) != 0),
+                           (key_params.flags & GS_FLAG_QUADRUPOLE) != 0, use),
                  measure, out);
     if (st != GS_OK) {
         gs_batch_set_shape(b, &keep);
