@@ -737,8 +737,8 @@ gs_status energy_f64(gs_sim* s, double* kinetic, double* potential) {
     return GS_OK;
 }
 
-// j-chunks of a plain launch: enough blocks for blocks_per_sm on every SM, at least 256
-// sources per chunk, at most 64 chunks
+// j-chunks that gs_set_shape judges a shape by: enough blocks for blocks_per_sm on every SM, at
+// least 256 sources per chunk, at most 64 chunks
 static int pick_chunks(uint64_t n_al, int ipt, uint32_t blocks_per_sm) {
     const uint64_t itiles = (n_al + kDirectBlock * ipt - 1) / (kDirectBlock * ipt);
     const uint64_t want_blocks = 152ull * blocks_per_sm;
@@ -787,12 +787,11 @@ ShapeUse direct_shape_use(const gs_params* p, uint64_t n_al) {
 }
 
 // Lays the j-chunk partials and tickets out in the system's slab (sizing pass: counts), for
-// the j-split of the creation shape.  direct_max_chunks keeps gs_set_shape's limit: a shape
-// may ask for no finer split than one laid out by pick_chunks would hold.
+// the j-split of the creation shape (a later shape's split is capped by it).
+// direct_max_chunks is gs_set_shape's limit and no scratch: what pick_chunks gives for the
+// creation shape, as callers of gs_set_shape know it.
 void direct_carve(gs_sim* s) {
     DirectWork& w = s->dw;
-    w.ipt = shape_ipt(s->shape);
-    w.block = kDirectBlock;
     const int c2 = pick_chunks(s->n_al, 2, s->shape.direct_blocks_per_sm);
     const int c4 = pick_chunks(s->n_al, 4, s->shape.direct_blocks_per_sm);
     s->direct_max_chunks = (uint32_t)(c2 > c4 ? c2 : c4);

@@ -152,8 +152,6 @@ struct BHWork {
 };
 
 struct DirectWork {
-    int ipt = 2;           // particles per thread of the creation shape
-    int block = 128;       // threads per block
     float4* partials = nullptr;  // [rows][N_al] {sx, sy, cx, cy}
     uint32_t* tickets = nullptr; // [i-tiles]
     uint32_t rows = 0;           // j-chunks the partials hold (0, 1: no partials)
@@ -267,7 +265,7 @@ struct gs_sim {
     uint32_t launches_per_step[4] = {0, 0, 0, 0};  // per graph (replay count)
     bool amag_known = false;         // relative criterion: every particle has its previous |a|
     gs_shape shape{};                // launch shapes (gs_set_shape; graphs are captured with them)
-    uint32_t direct_max_chunks = 1;  // j-chunks the direct-sum scratch was laid out for
+    uint32_t direct_max_chunks = 1;  // finest j-split that gs_set_shape accepts (direct sum)
     uint64_t kernel_launches = 0;    // kernels launched since creation
     void* slab = nullptr;            // every device buffer of the system
     size_t carved = 0;               // bytes laid out so far (sim_carve)
@@ -387,7 +385,7 @@ bool force_shape_supported(uint32_t warps, uint32_t short_lists);
 // batched stages (one launch per stage over every system of a plan)
 void bh_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& shape);
 void direct_batch_desc(gs_sim* s, SysDesc& d, uint32_t blocks[kTabCount], const gs_shape& batch_shape);
-// j-chunks the direct sum of `s` splits into under a shape (its scratch holds direct_max_chunks)
+// j-chunks that gs_set_shape judges a shape of `s` by (at most direct_max_chunks are accepted)
 uint32_t direct_chunks_needed(const gs_sim* s, const gs_shape& sh);
 int bh_batch_force_grid(const BatchPlan& p);
 // A second stream and two events: the moment prefix of the quadrupole mode runs there,
