@@ -59,7 +59,7 @@ ERROR_SAMPLE = 16384  # particles whose FP64 force the gated error is measured o
 # DRAM bytes of one launch of the traversal kernel on a workload, from an ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum), and that launch's algorithmic bytes
 FORCE_CAPTURE = {
-    "bh500k": {"traffic": 55.191040e6 + 1.843712e6, "algorithmic": 49.034368e6},
+    "bh500k": {"traffic": 55.077120e6 + 2.681088e6, "algorithmic": 49.034368e6},
 }
 
 
@@ -717,7 +717,8 @@ def roofline_of(gsim, wl, m, capture=None):
         t = m["stage_ms"]["direct"] / 1e3
         n_al = (wl["n"] + 63) // 64 * 64
         achieved = 14.0 * n_al * n_al / t / 1e12
-        extra = {"kernel": "k_direct_fast", "pairs_per_step": n_al * n_al, "flop_model": "14 FLOP per pair"}
+        extra = {"kernel": "k_direct_small" if n_al <= 12288 else "k_direct_fast", "pairs_per_step": n_al * n_al,
+                 "flop_model": "14 FLOP per pair"}
     traffic = source = None
     if capture and algorithmic:
         traffic = capture["traffic"] * algorithmic / capture["algorithmic"]

@@ -525,9 +525,10 @@ SortPassFn sort_pass_kernel_kpt(bool identity, uint32_t lb) {
     }
 }
 // Keys per thread of a system sorted alone.  A tile's ranks are a serial chain over a thread's
-// keys, and up to kSortSmallMax keys the look-back over the tiles is one round trip however
-// small they are, so a small system takes tiles of 1024 keys whatever its shape says (three
-// passes over 10,000 keys: 22 us, in tiles of 4096 32; over 100,000: 26 and 36).
+// keys, so a small system takes tiles of 1024 keys whatever its shape says.  The look-back takes
+// ceil(tiles / width) round trips, at most four at kSortSmallMax keys and 32 tiles a trip, and
+// costs less than the shorter chains gain (three passes over 10,000 keys: 22 us, in tiles of 4096
+// 32; over 100,000: 26 and 36).
 constexpr uint64_t kSortSmallMax = 131072;
 inline uint32_t sort_kpt(uint64_t n, const gs_shape& sh) {
     return n <= kSortSmallMax ? 4u : sh.sort_keys_per_thread == 8 ? 8u : 16u;
@@ -1898,7 +1899,7 @@ cudaError_t bh_step(gs_sim* s, int in, int out, bool profile, bool estimate) {
     }
     stage_end(s, kStageRecords, profile);
     stage_begin(s, kStageSums, profile);
-    if (!w.quad && !small) {  // monopole moments, level by level (the quadrupole mode has them from k_nodes)
+    if (!w.quad && !small) {  // monopole moments, level by level (the quadrupole mode has them from k_mom_nodes)
         const int safe = (s->p.flags & GS_FLAG_SAFE_RADIUS) ? 1 : 0;
         const int bb = bbox ? 1 : 0;
         const int per_sm = (int)s->shape.moment_blocks_per_sm < w.sums_per_sm ? (int)s->shape.moment_blocks_per_sm

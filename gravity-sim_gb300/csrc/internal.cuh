@@ -28,7 +28,7 @@ constexpr int kBBoxMaxBits = 15;            // largest per-axis bits (30-bit key
 constexpr uint32_t kKeyRemovedSort = 1u << 20;  // sort key of removed particles (fixed box)
 // Relative criterion: costly groups are walked by warp pairs in systems of at least this
 // many (padded) particles -- more groups than the traversal keeps resident at once, where
-// the longest walks trail the launch; smaller systems walk every group on one warp.
+// the longest walks trail the launch.
 constexpr uint32_t kHeavyMinParticles = 1u << 18;
 constexpr uint32_t kKeyRemoved = 0xFFFFFFFFu;   // reported key of removed particles
 
@@ -46,16 +46,18 @@ constexpr int kErrScanWait = 2;
 constexpr int kErrTree = 4;
 constexpr int kErrBarrierWait = 8;
 
-// radix sort: 256 threads x 8 or 16 keys per tile (gs_shape.sort_keys_per_thread)
+// radix sort: 256 threads x 8 or 16 keys per tile (gs_shape.sort_keys_per_thread), or 4 in a
+// small system sorted alone
 constexpr int kSortThreads = 256;
 // single-pass scan shape
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 // moments: levels at or above kLevelTop (<= 341 nodes) are summed by one block, every
-// deeper level by a launch of its own
+// deeper level by the whole grid (a batch: by a launch of its own)
 constexpr int kLevelTop = 4;
-// bounded spin for decoupled look-back: after this many polls the kernel flags an error
+// bounded spin of every device wait (look-back, grid barrier, the hand-over between two warps of
+// a walk): after this many polls the kernel flags an error
 constexpr uint32_t kSpinLimit = 1u << 24;
 
 // Order-preserving code of a float: unsigned comparison of the words orders the values

@@ -157,7 +157,7 @@ gs_status device_error(int err) {
     if (err) {
         set_error(std::string("device-side error flags ") + std::to_string(err) +
                   " (1: radix-sort look-back wait ran out, 2: scan look-back wait ran out, 4: tree capacity, "
-                  "8: moments grid barrier wait ran out)");
+                  "8: a wait of the moments grid barrier or between the two warps of a walk ran out)");
         return GS_ERR_DEVICE;
     }
     return GS_OK;

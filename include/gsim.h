@@ -140,16 +140,26 @@ typedef struct gs_sim gs_sim;
  * src/Simulation/Direct/DirectSimulation.cpp:9); here each system gets a shape from the
  * tuned table (gs_tune_shape) or the defaults, and gs_set_shape can change it between
  * steps.  No field changes a result bit, except direct_blocks_per_sm in FAST math, which
- * sets how the direct sum splits its j-range over blocks (and so its summation grouping). */
+ * sets how the direct sum splits its j-range over blocks (and so its summation grouping).
+ * A system run alone does not read a field where its size has kernels of its own:
+ *   - the sort, scan and moments fields up to 8,192 padded particles (3,072 in quadrupole mode),
+ *     whose tree is built in one block;
+ *   - sort_keys_per_thread up to 131,072 (tiles of 1024 keys);
+ *   - moment_blocks_per_sm up to about 313,000 (fewer blocks than one an SM);
+ *   - the direct-sum fields up to 12,288 and in REFERENCE math.
+ * A batch reads the sort, scan and force fields of its own shape at every size, and
+ * direct_targets for direct sums above 12,288. */
 typedef struct gs_shape {
     uint32_t sort_keys_per_thread; /* radix-sort tile = 256 threads x this: 8 or 16 (default) */
     uint32_t sort_lookback;        /* earlier tiles a radix pass reads per look-back round trip: 8, 16, 32 */
     uint32_t scan_lookback;        /* the same for the node scan: 32, 64, 128 */
     uint32_t force_warps;          /* group walks per block of the accurate traversal: 1, 2 (default), 4;
                                       1 runs as 2 where costly groups are walked by warp pairs */
-    uint32_t force_short_lists;    /* 0: evaluate after 160 nodes / 96 leaf runs; 1: after 96 / 64 */
+    uint32_t force_short_lists;    /* 0: a walk's lists are summed beyond 128 nodes or 64 leaf runs (63 of
+                                      either where two warps share a walk); 1: beyond 64 / 32 (31) */
     uint32_t direct_targets;       /* direct-sum particles per thread (FAST math): 2 (default) or 4 */
-    uint32_t direct_blocks_per_sm; /* direct-sum j-split target, blocks per SM: 1..32 (default 12) */
+    uint32_t direct_blocks_per_sm; /* direct-sum j-split target, blocks per SM: 1..32 (default 12); at most
+                                      the split that the creation shape laid scratch out for */
     uint32_t moment_blocks_per_sm; /* blocks per SM of the cooperative moments launch of the monopole
                                       mode: 1 or 2 (default); the quadrupole mode has no such launch */
 } gs_shape;
@@ -188,8 +198,9 @@ GS_API gs_status gs_run(gs_sim* sim, uint32_t count);
 /* Wait for all submitted steps; timeout_ns = 0 uses the system's timeout. */
 GS_API gs_status gs_sync(gs_sim* sim, uint64_t timeout_ns);
 /* The system's launch shapes; changing them drops its captured step graphs.  A
- * direct_blocks_per_sm that needs more j-chunk scratch than gs_create laid out is refused
- * (GS_ERR_CAPACITY). */
+ * direct_blocks_per_sm far above the creation shape's is refused (GS_ERR_CAPACITY): one that
+ * would split the sources, in chunks of at least 256, into more chunks than the creation
+ * shape's value with 2 or 4 targets per thread. */
 GS_API gs_status gs_get_shape(gs_sim* sim, gs_shape* out);
 GS_API gs_status gs_set_shape(gs_sim* sim, const gs_shape* shape);
 GS_API void gs_shape_defaults(gs_shape* out);
@@ -262,10 +273,11 @@ GS_API uint64_t gs_bh_node_capacity(int32_t box_mode, uint64_t aligned_count);
  *   - Runs on the calling thread's current device, on `stream` (a cudaStream_t, NULL for
  *     the legacy default stream), asynchronously.
  *   - Scratch lives in fixed device arrays inside this library (about 4 MiB per GPU that
- *     loads it, held until the process exits).  Every call looks up their device
- *     addresses in the current context (no allocation); the first call on a device also
- *     loads the library's module there, so make it before any stream capture.
- *   - Every call shares those arrays: calls that overlap on the GPU (other streams,
+ *     loads it, held until the process exits).  A call above 12,288 particles looks up their
+ *     device addresses in the current context (no allocation; smaller ones need no scratch);
+ *     the first call on a device also loads the library's module there, so make it before any
+ *     stream capture.
+ *   - The calls share those arrays: calls that overlap on the GPU (other streams,
  *     other threads) race and give wrong results.  Serialise them on one stream. */
 #define GS_NOALLOC_MAX_PARTICLES 65536
 GS_API gs_status gs_direct_step_noalloc(const float* d_pos_in, const float* d_vel_in,
@@ -322,7 +334,8 @@ GS_API gs_status gs_tune_crossover(const gs_params* direct_params, const gs_para
  *
  * gs_tune_shape times candidate gs_shape values on a system of n particles made by
  * gs_generate(generator, seed) with these parameters, and keeps the fastest: coordinate
- * descent over the knobs that apply (Barnes-Hut: sort tile, sort and scan look-back
+ * descent over the knobs that apply (a field that a system of this size does not read, see
+ * gs_shape, is timed but keeps its default; Barnes-Hut: sort tile, sort and scan look-back
  * widths, group-walk warps per block and list caps, moments grid; direct sum: targets per
  * thread and the j-split), each candidate timed with CUDA events as the median of `steps`
  * warm steps with the L2 flushed before each.  The winner goes into the process's tuned

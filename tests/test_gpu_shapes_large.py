@@ -1,5 +1,5 @@
 """Launch shapes at sizes whose kernels read every field: trees above 8,192 (3,072 with
-quadrupoles) particles, sort tiles above 131,072, the moments launch above 311,296, direct sums
+quadrupoles) particles, sort tiles above 131,072, the moments launch from 313,344, direct sums
 above 12,288.  Barnes-Hut in REFERENCE math bit-identical to the oracle, direct sums as with the
 other number of targets per thread, members of a batch as alone."""
 import itertools
